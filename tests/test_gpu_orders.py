@@ -1,0 +1,80 @@
+"""The one-point-per-block FP64 kernels at the edges of their tile splits.
+
+Orders just below, at and above each padded order (8, 16, 24, 32, 48), leads
+of another order than the device, layers with their own blocks, and both tile
+splits of order 9..16 (chosen by the number of points).  Random systems at an
+eta that keeps the decimation well conditioned, against the CPU oracle to the
+parity bound of the FP64 path, 1e-10 of the largest entry.
+"""
+
+import numpy as np
+import pytest
+import torch
+
+from negfpy_b200 import engine
+from oracle import negf_oracle as O
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-10
+ETA = 0.05
+
+
+def _herm(rng, n):
+    a = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))
+    return (a + a.conj().T) / (2 * np.sqrt(n)) + 2.0 * np.eye(n)
+
+
+def _any(rng, n, m):
+    return 0.6 * (rng.standard_normal((n, m)) + 1j * rng.standard_normal((n, m))) / np.sqrt(n + m)
+
+
+def _system(n, nl, nr, layers, seed):
+    rng = np.random.default_rng(seed)
+    lead = lambda m: (_herm(rng, m), _any(rng, m, m))  # noqa: E731
+    return {"l": lead(nl), "r": lead(nr), "on": [_herm(rng, n) for _ in range(layers)],
+            "cp": [_any(rng, n, n) for _ in range(layers - 1)], "vl": _any(rng, n, nl), "vr": _any(rng, n, nr)}
+
+
+def _solve(s, omegas):
+    c = lambda x: x[None]  # noqa: E731
+    lead = lambda b: {"d00": c(b[0]), "d01": c(b[1]), "d10": None}  # noqa: E731
+    cp = np.stack(s["cp"]) if s["cp"] else np.zeros((1,) + s["on"][0].shape, dtype=complex)
+    sysobj = engine.StackedSystem.from_arrays(lead(s["l"]), lead(s["r"]), np.stack(s["on"])[None], cp[None],
+                                              len(s["on"]), s["vl"][None], s["vr"][None], same_leads=False)
+    om = torch.as_tensor(omegas, device="cuda")
+    ki = torch.zeros(om.numel(), dtype=torch.int32, device="cuda")
+    eta = torch.full_like(om, ETA)
+    g = engine.sgf_sr(*sysobj.lead_l, om, eta, ki, want_dos=True)
+    r = sysobj.transmission(om, ki, eta)
+    assert int(r["status"].abs().sum()) == 0 and int(g["status"].abs().sum()) == 0
+    return g["g"].cpu().numpy(), g["dos"].cpu().numpy(), r["T"].cpu().numpy(), g["iters"].cpu().numpy()
+
+
+@pytest.mark.parametrize("n,nl,nr,layers", [
+    (2, 2, 2, 3), (7, 8, 7, 1), (8, 8, 3, 4), (9, 9, 9, 2), (15, 16, 2, 3), (16, 16, 16, 3), (17, 17, 9, 2),
+    (23, 24, 23, 3), (24, 24, 24, 1), (25, 25, 8, 2), (31, 32, 31, 2), (32, 32, 32, 3), (33, 33, 25, 2),
+    (40, 40, 41, 2), (47, 48, 47, 3), (48, 48, 48, 2), (5, 48, 20, 2)])
+def test_orders_match_oracle(n, nl, nr, layers):
+    s = _system(n, nl, nr, layers, seed=100 * n + nl)
+    omegas = np.array([0.3, 1.1, 1.9])
+    g, dos, t, it = _solve(s, omegas)
+    for i, w in enumerate(omegas):
+        ref, nit = O.sancho_rubio(w, *s["l"], None, ETA)
+        assert it[i] == nit
+        assert np.max(np.abs(g[i] - ref)) <= TOL * np.max(np.abs(ref))
+        d = O.lead_surface_dos(w, *s["l"], None, ETA)
+        assert abs(dos[i] - d) <= 10 * TOL * max(abs(d), 1.0)
+        tr = O.transmission_point(w, s["on"], s["cp"], (*s["l"], None), (*s["r"], None), ETA, vl=s["vl"], vr=s["vr"],
+                                  idx_l=np.arange(n), idx_r=np.arange(n * (layers - 1), n * layers))
+        assert abs(t[i] - tr) <= TOL * max(abs(tr), 1.0)
+
+
+@pytest.mark.parametrize("n", [9, 12, 16])
+def test_both_splits_of_order_16_agree_bitwise(n):
+    s = _system(n, n, n, 4, seed=n)
+    omegas = np.linspace(0.1, 2.5, 1200)  # above the few-points split, whose largest call is 592
+    g, dos, t, it = _solve(s, omegas)
+    for a, b in ((0, 592), (592, 593), (600, 1193)):
+        gp, dp, tp, ip = _solve(s, omegas[a:b])
+        for x, y in ((g, gp), (dos, dp), (t, tp), (it, ip)):
+            assert np.array_equal(x[a:b], y)
