@@ -99,7 +99,18 @@ int sr_f64_launch(const SrArgs& a, cudaStream_t st);
 // Padded order np = padded_order(max(n, nl, nr)) selects the kernel variant.
 int rgf_f64_grid(int np);  // persistent grid size (blocks), 0 for the 1x1 path
 int rgf_f64_launch(const RgfArgs& a, int np, int grid, cudaStream_t st);
-// Block orders 49..256 (padded to a multiple of 16): global-memory workspace kernels.
+// Block orders 49..104 (padded to a multiple of 8): one matrix in registers, one
+// operand in shared memory.
+namespace mid {
+constexpr int kMaxOrder = 104;
+int sr_grid(int np);
+int rgf_grid(int np);
+size_t sr_ws_bytes(int np, int grid);
+size_t rgf_ws_bytes(int np, int n, int grid);
+int sr_launch(const SrArgs& a, int np, int grid, double2* ws, unsigned* counter, cudaStream_t st);
+int rgf_launch(const RgfArgs& a, int np, int grid, double2* ws, cudaStream_t st);
+}  // namespace mid
+// Block orders 49..256 (those above 104 padded to a multiple of 16): global-memory workspace.
 int global_order(int n);  // padded order for n > 48, 0 if unsupported
 int sr_global_grid(int np);
 int rgf_global_grid(int np);

@@ -1,9 +1,9 @@
-// FP64 kernels for block orders 49..256 (padded to NP, a multiple of 16).
+// FP64 kernels for block orders 105..256 (padded to NP, a multiple of 16), and
+// the adjoint and full-G kernels of every order up to 256.
 //
-// One point's matrices do not fit one SM's shared memory beyond n = 48, so
-// here they live in a per-block workspace in global memory (mostly L2
-// resident) and the blocks are persistent: each takes points from an atomic
-// counter.  The decimation and sweep kernels are register-capped for two
+// Beyond n = 104 a block's registers do not hold a matrix, so here all of them
+// live in a per-block workspace in global memory (mostly L2 resident) and the
+// blocks are persistent: each takes points from an atomic counter.  The decimation and sweep kernels are register-capped for two
 // resident blocks per SM (128 registers a thread, a few hundred bytes of
 // spill), so one point's latency-bound pivot steps overlap another's
 // products: 1.22x (decimation) and 1.33x (sweep) faster at n = 96 than one
@@ -704,13 +704,23 @@ static int occupancy_grid(K kernel, int np) {
 
 }  // namespace glob
 
-int sr_global_grid(int np) { return glob::occupancy_grid(glob::sr_f64_global_kernel, np); }
-int rgf_global_grid(int np) { return glob::occupancy_grid(glob::rgf_f64_global_kernel, np); }
-size_t sr_global_ws_bytes(int np, int grid) { return (size_t)grid * 7 * np * np * 16; }
-size_t rgf_global_ws_bytes(int np, int n, int grid) { return (size_t)grid * (6 * (size_t)np * np + 2 * (size_t)n * n) * 16; }
+int sr_global_grid(int np) {
+  return np <= mid::kMaxOrder ? mid::sr_grid(np) : glob::occupancy_grid(glob::sr_f64_global_kernel, np);
+}
+int rgf_global_grid(int np) {
+  return np <= mid::kMaxOrder ? mid::rgf_grid(np) : glob::occupancy_grid(glob::rgf_f64_global_kernel, np);
+}
+size_t sr_global_ws_bytes(int np, int grid) {
+  return np <= mid::kMaxOrder ? mid::sr_ws_bytes(np, grid) : (size_t)grid * 7 * np * np * 16;
+}
+size_t rgf_global_ws_bytes(int np, int n, int grid) {
+  return np <= mid::kMaxOrder ? mid::rgf_ws_bytes(np, n, grid)
+                              : (size_t)grid * (6 * (size_t)np * np + 2 * (size_t)n * n) * 16;
+}
 
 int sr_f64_global_launch(const SrArgs& a, int np, int grid, double2* ws, unsigned* counter, cudaStream_t st) {
   if (a.batch <= 0) return 0;
+  if (np <= mid::kMaxOrder) return mid::sr_launch(a, np, grid, ws, counter, st);
   glob::sr_f64_global_kernel<<<grid, glob::kThreads, glob::smem_bytes(np), st>>>(a, np, ws, counter);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
@@ -761,6 +771,7 @@ int grad_f64_launch(const GradArgs& ga, int np, int grid, double2* ws, cudaStrea
 
 int rgf_f64_global_launch(const RgfArgs& a, int np, int grid, double2* ws, cudaStream_t st) {
   if (a.batch <= 0) return 0;
+  if (np <= mid::kMaxOrder) return mid::rgf_launch(a, np, grid, ws, st);
   glob::rgf_f64_global_kernel<<<grid, glob::kThreads, glob::smem_bytes(np), st>>>(a, np, ws);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
@@ -770,6 +781,6 @@ int rgf_f64_global_launch(const RgfArgs& a, int np, int grid, double2* ws, cudaS
 namespace negf {
 int global_order(int n) {
   if (n <= 48 || n > 256) return 0;
-  return (n + 15) / 16 * 16;
+  return n <= mid::kMaxOrder ? (n + 7) / 8 * 8 : (n + 15) / 16 * 16;
 }
 }  // namespace negf

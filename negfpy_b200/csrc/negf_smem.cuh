@@ -31,10 +31,15 @@ __device__ __forceinline__ double2 z_of(double w, double e) {
 }
 
 // NP: padded order; each warp owns TR x TC tiles of 8 x 8; OCC: thread blocks
-// per SM the registers are budgeted for.
-template <int NP_, int TR_, int TC_, int OCC_>
+// per SM the registers are budgeted for; KB: bits of the row index in a pivot
+// key (6 up to order 48, 8 above); LPR: lanes that share a panel row in the
+// pivot steps (0: as many as the threads allow); PARK: column tiles an
+// inversion keeps in Tensor Memory during the pivot steps (TR = 1 only), so
+// that these do not spill.
+template <int NP_, int TR_, int TC_, int OCC_, int KB_ = 6, int LPR_ = 0, int PARK_ = 0>
 struct Cfg {
-  static constexpr int NP = NP_, TR = TR_, TC = TC_, OCC = OCC_;
+  static constexpr int PARK = PARK_;
+  static constexpr int NP = NP_, TR = TR_, TC = TC_, OCC = OCC_, KB = KB_;
   static constexpr int T8 = NP / 8;
   static constexpr int WC = T8 / TC, WR = T8 / TR;
   static constexpr int NW = WR * WC;      // warps
@@ -43,7 +48,7 @@ struct Cfg {
   // A panel row is handled by LPR neighbouring lanes, EPT columns each: lane cl
   // has columns cl + LPR q.  Rows are PS elements apart, so that the rows of a
   // quarter warp fall into different banks.
-  static constexpr int LPR = NTH >= 8 * NP ? 8 : (NTH >= 4 * NP ? 4 : 2);
+  static constexpr int LPR = LPR_ ? LPR_ : (NTH >= 8 * NP ? 8 : (NTH >= 4 * NP ? 4 : 2));
   static constexpr int EPT = 8 / LPR;
   static constexpr int PS = LPR == 8 ? 8 : 8 + LPR;
   static constexpr int PE = NP * PS;      // complex elements of a panel
@@ -51,8 +56,9 @@ struct Cfg {
   // buffer (unused while a matrix is inverted) where it is large enough.
   static constexpr int SCR = 2 * PE + 8 * NP;
   static constexpr int BUF = MAT > SCR ? MAT : SCR;
-  static_assert(T8 % TR == 0 && T8 % TC == 0 && NP <= 64 && NW <= 32, "tile split");
-  static_assert(NTH >= 2 * NP && (NP * LPR) % 32 == 0, "panel rows per warp");
+  static_assert(T8 % TR == 0 && T8 % TC == 0 && NP <= (1 << KB) && NW <= 32, "tile split");
+  static constexpr int WW = (NP * LPR + 31) / 32;  // warps with panel rows
+  static_assert(WW <= NW, "panel rows per warp");
 };
 
 // Row-dependent XOR swizzle of the column index (bits 0-2), values
@@ -144,13 +150,9 @@ __device__ __forceinline__ void b_base(const Lane& L, int (&b)[2]) {
     b[h] = CT ? (L.C0 + L.g) * C::NP + (k ^ swz(L.g)) : k * C::NP + L.C0 + (L.g ^ swz(k));
   }
 }
-// Fragments of one row tile of A, of all the warp's column tiles of B.
+// Fragments of one row tile of A or one column tile of B.
 struct AFrag {
   double re[2], im[2];
-};
-template <class C>
-struct BFrag {
-  double re[C::TC][2], im[C::TC][2];
 };
 template <class C, bool CT>
 __device__ __forceinline__ void load_a(AFrag& f, const double2* S, const int (&b)[2], int kc, int i) {
@@ -163,29 +165,26 @@ __device__ __forceinline__ void load_a(AFrag& f, const double2* S, const int (&b
   }
 }
 template <class C, bool CT>
-__device__ __forceinline__ void load_b(BFrag<C>& f, const double2* S, const int (&b)[2], int kc) {
-  const int off = CT ? kc * 8 : kc * 8 * C::NP;
+__device__ __forceinline__ void load_b(AFrag& f, const double2* S, const int (&b)[2], int kc, int j) {
+  const int off = CT ? kc * 8 + 8 * j * C::NP : kc * 8 * C::NP + 8 * j;
 #pragma unroll
-  for (int j = 0; j < C::TC; ++j)
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const double2 v = S[b[h] + off + (CT ? 8 * j * C::NP : 8 * j)];
-      f.re[j][h] = v.x;
-      f.im[j][h] = CT ? -v.y : v.y;
-    }
+  for (int h = 0; h < 2; ++h) {
+    const double2 v = S[b[h] + off];
+    f.re[h] = v.x;
+    f.im[h] = CT ? -v.y : v.y;
+  }
 }
 // One chunk of 8 of one tile: re += ar br, then - ai bi; im += ar bi, then
 // ai br (each over its 8 terms in order, as one m16n8k8 per term pair would).
-template <class C>
-__device__ __forceinline__ void chunk(double (&re)[2], double (&im)[2], const AFrag& a, const BFrag<C>& b, int j) {
-  dmma(re, a.re[0], b.re[j][0]);
-  dmma(im, a.re[0], b.im[j][0]);
-  dmma(re, a.re[1], b.re[j][1]);
-  dmma(im, a.re[1], b.im[j][1]);
-  dmma(re, -a.im[0], b.im[j][0]);
-  dmma(im, a.im[0], b.re[j][0]);
-  dmma(re, -a.im[1], b.im[j][1]);
-  dmma(im, a.im[1], b.re[j][1]);
+__device__ __forceinline__ void chunk(double (&re)[2], double (&im)[2], const AFrag& a, const AFrag& b) {
+  dmma(re, a.re[0], b.re[0]);
+  dmma(im, a.re[0], b.im[0]);
+  dmma(re, a.re[1], b.re[1]);
+  dmma(im, a.re[1], b.im[1]);
+  dmma(re, -a.im[0], b.im[0]);
+  dmma(im, a.im[0], b.re[0]);
+  dmma(re, -a.im[1], b.im[1]);
+  dmma(im, a.im[1], b.re[1]);
 }
 
 // c1 = op(A1) op(B) and, with two left operands, c2 = op(A2) op(B), over the
@@ -200,9 +199,9 @@ __device__ __forceinline__ void mm_(Acc<C>& c1, Acc<C>& c2, const double2* A1, c
   b_base<C, BC>(L, bb);
   c1.zero();
   if (NA == 2) c2.zero();
-  AFrag a, an;
-  BFrag<C> b, bn;
-  load_b<C, BC>(b, B, bb, 0);
+  AFrag a, an, b[C::TC], bn[C::TC];
+#pragma unroll
+  for (int j = 0; j < C::TC; ++j) load_b<C, BC>(b[j], B, bb, 0, j);
   load_a<C, AC>(a, A1, ab, 0, 0);
 #pragma unroll 1
   for (int kc = 0; kc < kch; ++kc) {
@@ -212,13 +211,17 @@ __device__ __forceinline__ void mm_(Acc<C>& c1, Acc<C>& c2, const double2* A1, c
       const int i = r % C::TR, rn = r + 1;
       if (rn < NA * C::TR) load_a<C, AC>(an, rn < C::TR ? A1 : A2, ab, kc, rn % C::TR);
       else load_a<C, AC>(an, A1, ab, kn, 0);
-      if (r == 0) load_b<C, BC>(bn, B, bb, kn);
+      if (r == 0) {
+#pragma unroll
+        for (int j = 0; j < C::TC; ++j) load_b<C, BC>(bn[j], B, bb, kn, j);
+      }
       Acc<C>& c = r < C::TR ? c1 : c2;
 #pragma unroll
-      for (int j = 0; j < C::TC; ++j) chunk<C>(c.re[i][j], c.im[i][j], a, b, j);
+      for (int j = 0; j < C::TC; ++j) chunk(c.re[i][j], c.im[i][j], a, b[j]);
       a = an;
     }
-    b = bn;
+#pragma unroll
+    for (int j = 0; j < C::TC; ++j) b[j] = bn[j];
   }
 }
 template <class C, bool AC, bool BC>
@@ -253,260 +256,6 @@ __device__ __forceinline__ double2 crecip_smith(double2 v) {
   const double r = v.x / v.y;
   const double i = 1.0 / fma(v.x, r, v.y);
   return make_double2(r * i, -i);
-}
-
-// ---------------------------------------------------------- Gauss-Jordan --
-template <class C>
-struct GJ {
-  alignas(16) double2 lam[2];          // the panel's scale, double-buffered by column parity
-  alignas(16) unsigned key[8][C::NW];  // each warp's pivot key of each panel column
-  int newpos[C::NP];                   // position after the panel of each panel row
-  int cmapinv[C::NP];
-};
-
-// Pivot key of a candidate entry: top bits of max(|re|, |im|) with the row
-// index (< 64) in the low 6 bits, so the unsigned maximum over a column picks
-// the largest entry up to a relative 2^-14, ties to the lowest row.
-__device__ __forceinline__ unsigned pivot_key(double2 v, int r) {
-  return (hi_word(v) & ~63u) | (unsigned)(63 - r);
-}
-
-// Inverse of the matrix held in m (leading n x n block, identity padding) by
-// blocked Gauss-Jordan elimination with partial pivoting, into the shared
-// matrix out; scr (SCR complex, may be out itself) is scratch.  Ends with the
-// block synchronised.
-//
-// Columns are processed in panels of 8.  The n x 8 panel is factored in shared
-// memory by the whole block with one barrier per column and no division: it is
-// kept as W = lambda P (P the textbook Gauss-Jordan panel, lambda a complex
-// scalar) and, with p the pivot and s a power of two bringing p near 1,
-//     new(r, c) = (p s) a' - (s b') m,   lambda <- lambda p s
-//     a' = 0 if r is the pivot row or c the pivot column, else W(r, c)
-//     b' = -lambda for the pivot row, else W(r, j)
-//     m  =  lambda for the pivot column, else W(pivot row, c)
-// (expanding W = lambda P gives the textbook update times the new lambda;
-// |p s| lies in [1, 2.83]).  Pivot search is looked ahead: the threads that
-// write column j+1 of the panel reduce its pivot keys (see pivot_key) over the
-// rows not yet used as pivots, one slot per warp, before the barrier; the key's
-// exponent bits give s.
-//
-// The matrix itself never moves: a thread keeps its elements in registers for
-// the whole inversion and only tracks the position of its rows.  It writes its
-// part of the panel's 8 columns to shared memory at those positions, and its
-// part of the pivot rows once they are known; the rank-8 update then
-// accumulates in place on the tensor path,
-//     row r, columns Q: [r not a pivot row] W(r, Q) + P(r, :) W(pivot rows, Q),
-//     row r, panel:     P(r, :),                      P = W / lambda.
-// The row order and the undone column interchanges (column c of the inverse is
-// column t_{n-1}(...t_0(c)) of the eliminated matrix, t_k = (k b_k), b_k the
-// position of the k-th pivot) are applied as the result is written.  Keeping
-// the matrix in registers instead of two shared buffers removes its reload and
-// rewrite in each of the n/8 updates and is what lets several points share an SM.
-// Returns kOk, kSingular (all candidates zero or below 2^-1022) or kNonFinite
-// identically in every thread.
-template <class C>
-__device__ __forceinline__ int gj_invert(Acc<C>& m, double2* scr, double2* out, int n, const Lane& L, GJ<C>& sh) {
-  constexpr int PE = C::PE, NP = C::NP, NW = C::NW;
-  constexpr int LPR = C::LPR, EPT = C::EPT, PS = C::PS;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const bool work = C::NTH == NP * LPR || tid < NP * LPR;  // whole warps
-  const int pr_own = work ? tid / LPR : 0, cl = tid % LPR;
-  const int prow = pr_own * PS;
-  double2* const Bp = scr + 2 * PE;  // the panel's pivot rows [8][NP]
-  int pos[C::TR];  // position of each of the thread's matrix rows
-#pragma unroll
-  for (int i = 0; i < C::TR; ++i) pos[i] = L.r0 + 8 * i;
-  // The last warp (without panel rows where the block has warps to spare)
-  // keeps lambda and the permutations: lane l those of rows and columns l,
-  // l + 32.
-  const bool bk = warp == NW - 1;
-  constexpr bool kSpare = C::NTH > NP * LPR;
-  constexpr int RL = (NP + 31) / 32;
-  int cm[RL];  // t_k(...t_0(c)) over the steps done so far
-#pragma unroll
-  for (int i = 0; i < RL; ++i) cm[i] = lane + 32 * i;
-
-#pragma unroll 1
-  for (int k0 = 0, par = 0; k0 < n; k0 += 8, par ^= 1) {
-    const int jmax = (n - k0) < 8 ? (n - k0) : 8;
-    // A full panel's 8 steps end in the buffer they began in, so the next
-    // panel starts in the other one while this one may still be read.
-    double2* const P0 = scr + par * PE;
-    double2* const P1 = scr + (par ^ 1) * PE;
-    const int pj = (k0 - L.C0) >> 3;  // the panel's tile column among the thread's, if in range
-    // ---- publish the panel, keys of panel column 0 ----
-    unsigned key0 = 0u;
-#pragma unroll
-    for (int j = 0; j < C::TC; ++j)
-      if (j == pj) {
-#pragma unroll
-        for (int i = 0; i < C::TR; ++i) {
-          double2* row = P0 + pos[i] * PS + 2 * L.t;
-          row[0] = m.get(i, j, 0);
-          row[1] = m.get(i, j, 1);
-          if (L.t == 0 && pos[i] >= k0 && pos[i] < n) key0 = max(key0, pivot_key(m.get(i, j, 0), pos[i]));
-        }
-      }
-    key0 = __reduce_max_sync(0xffffffffu, key0);
-    if (lane == 0) sh.key[0][warp] = key0;
-    if (tid == 0) sh.lam[0] = make_double2(1.0, 0.0);
-    __syncthreads();
-    // ---- factor the panel, one barrier per column ----
-    double2 av[EPT];  // this thread's panel elements
-#pragma unroll
-    for (int q = 0; q < EPT; ++q) av[q] = P0[prow + cl + LPR * q];
-    bool cand = work && pr_own >= k0 && pr_own < n;  // row not yet a pivot
-    int lg[RL];                                      // position of panel rows lane, lane + 32
-#pragma unroll
-    for (int i = 0; i < RL; ++i) lg[i] = lane + 32 * i;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      if (j >= jmax) break;
-      const double2* Pc = (j & 1) ? P1 : P0;
-      double2* Pn = (j & 1) ? P0 : P1;
-      // What does not depend on the pivot is loaded with the key, whose slots
-      // are read one lane per slot.
-      const double2 fv = Pc[prow + j];
-      const double2 lam = sh.lam[j & 1];
-      unsigned key;
-      if (NW == 4) {
-        const uint4 kv = *reinterpret_cast<const uint4*>(sh.key[j]);
-        key = max(max(kv.x, kv.y), max(kv.z, kv.w));
-      } else if (NW == 2) {
-        const uint2 kv = *reinterpret_cast<const uint2*>(sh.key[j]);
-        key = max(kv.x, kv.y);
-      } else if (NW == 1) {
-        key = sh.key[j][0];
-      } else {
-        key = __reduce_max_sync(0xffffffffu, lane < NW ? sh.key[j][lane] : 0u);
-      }
-      // A zero or non-finite pivot ends the inversion at the end of this step
-      // (off the path to the pivot row); min keeps its row in the panel.
-      const bool stop = key - 64u >= 0x7ff00000u - 64u;
-      const int pr = min(63 - (int)(key & 63u), NP - 1);
-      const int ex = (int)(key >> 20);
-      const double sc = (ex != 0 && ex < 2046) ? __hiloint2double((2046 - ex) << 20, 0) : 1.0;
-      const double2* prow_p = Pc + pr * PS;
-      const double2 piv = prow_p[j];
-      const double2 ps = make_double2(piv.x * sc, piv.y * sc);
-      unsigned nk = 0u;
-      if (work) {
-        double2 mv[EPT];
-#pragma unroll
-        for (int q = 0; q < EPT; ++q) mv[q] = prow_p[cl + LPR * q];
-        const bool isp = pr_own == pr;
-        cand = cand && !isp;
-        const double2 bb = isp ? cneg(lam) : fv;
-        const double2 b = make_double2(bb.x * sc, bb.y * sc);
-        // The next pivot column first, so that its keys are reduced under the
-        // other columns' updates.
-#pragma unroll
-        for (int qq = 0; qq < EPT; ++qq) {
-          const int q = (qq + (j + 1) / LPR) % EPT;
-          const int c = cl + LPR * q;
-          const bool pivcol = q == j / LPR && cl == j % LPR;
-          double2 v = cneg(cmul(b, pivcol ? lam : mv[q]));
-          if (!isp && !pivcol) cfma(v, ps, av[q]);
-          Pn[prow + c] = v;
-          av[q] = v;
-          if (j + 1 < 8 && qq == 0) {
-            if (cl == (j + 1) % LPR && cand) nk = pivot_key(v, pr_own);
-            nk = __reduce_max_sync(0xffffffffu, nk);
-          }
-        }
-      }
-      if (j + 1 < 8 && lane == 0) sh.key[j + 1][warp] = nk;
-      if (bk) {
-        double2 ln = cmul(lam, ps);
-        if (kSpare && j == 7) ln = crecip_smith(ln);  // under the other warps' element updates
-        if (lane == 0) sh.lam[(j + 1) & 1] = ln;
-        // the row interchange of this step: positions k and bl
-        const int k = k0 + j;
-        int x = lg[0];
-        if (RL == 2) x = pr & 32 ? lg[RL - 1] : x;
-        const int bl = __shfl_sync(0xffffffffu, x, pr & 31);
-#pragma unroll
-        for (int i = 0; i < RL; ++i) {
-          lg[i] = lane + 32 * i == pr ? k : (lg[i] == k ? bl : lg[i]);
-          cm[i] = cm[i] == k ? bl : (cm[i] == bl ? k : cm[i]);
-          if (j + 1 == jmax && lane + 32 * i < NP) sh.newpos[lane + 32 * i] = lg[i];
-        }
-      }
-      if (stop) return (key >> 6) == 0u ? kSingular : kNonFinite;
-      __syncthreads();
-    }
-    // ---- rank-8 update in registers ----
-    // The owners of the pivot rows hand out their elements before the panel.
-    int np[C::TR];
-#pragma unroll
-    for (int i = 0; i < C::TR; ++i) np[i] = sh.newpos[pos[i]];
-#pragma unroll
-    for (int i = 0; i < C::TR; ++i) {
-      if ((unsigned)(np[i] - k0) < (unsigned)jmax) {
-        double2* row = Bp + (np[i] - k0) * NP;
-        const int sw = swz(np[i]);
-#pragma unroll
-        for (int j = 0; j < C::TC; ++j)
-#pragma unroll
-          for (int q = 0; q < 2; ++q) {
-            row[L.C0 + 8 * j + ((2 * L.t + q) ^ sw)] = m.get(i, j, q);
-            m.set(i, j, q, make_double2(0.0, 0.0));
-          }
-      }
-    }
-    const double2* P = (jmax & 1) ? P1 : P0;
-    const double2 ll = sh.lam[jmax & 1];
-    const double2 il = kSpare && jmax == 8 ? ll : crecip_smith(ll);
-    AFrag a[C::TR];
-#pragma unroll
-    for (int i = 0; i < C::TR; ++i)
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const double2 v = cmul(P[pos[i] * PS + L.t + 4 * h], il);
-        a[i].re[h] = v.x;
-        a[i].im[h] = v.y;
-      }
-    __syncthreads();
-    BFrag<C> b;
-#pragma unroll
-    for (int j = 0; j < C::TC; ++j)
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int kk = L.t + 4 * h;
-        const double2 v = Bp[sidx<NP>(kk, L.C0 + 8 * j + L.g)];
-        b.re[j][h] = kk < jmax ? v.x : 0.0;
-        b.im[j][h] = kk < jmax ? v.y : 0.0;
-      }
-#pragma unroll
-    for (int j = 0; j < C::TC; ++j) {
-      if (j == pj) {  // the panel's columns take P(r, :) (warp-uniform)
-#pragma unroll
-        for (int i = 0; i < C::TR; ++i)
-#pragma unroll
-          for (int q = 0; q < 2; ++q) m.set(i, j, q, cmul(P[pos[i] * PS + 2 * L.t + q], il));
-      } else {
-#pragma unroll
-        for (int i = 0; i < C::TR; ++i) chunk<C>(m.re[i][j], m.im[i][j], a[i], b, j);
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < C::TR; ++i) pos[i] = np[i];
-  }
-  if (bk)
-#pragma unroll
-    for (int i = 0; i < RL; ++i)
-      if (lane + 32 * i < NP) sh.cmapinv[cm[i]] = lane + 32 * i;
-  __syncthreads();  // the last panel and its pivot rows are read, cmapinv is complete
-#pragma unroll
-  for (int j = 0; j < C::TC; ++j)
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      const int c = sh.cmapinv[L.c0 + 8 * j + q];
-#pragma unroll
-      for (int i = 0; i < C::TR; ++i) out[sidx<NP>(pos[i], c)] = m.get(i, j, q);
-    }
-  __syncthreads();
-  return kOk;
 }
 
 // ---------------------------------------------------- thread-private matrices --
@@ -552,6 +301,322 @@ __device__ __forceinline__ void tmem_get(uint32_t addr, double2 (&v)[N][2]) {
       v[i][q] = make_double2(__hiloint2double(r[i][4 * q + 1], r[i][4 * q]),
                              __hiloint2double(r[i][4 * q + 3], r[i][4 * q + 2]));
   }
+}
+
+// f(j, elements) for tiles 0 .. N-1 at consecutive addresses, four in flight.
+template <int N, class F>
+__device__ __forceinline__ void tmem_tiles(uint32_t addr, F&& f) {
+#pragma unroll
+  for (int j = 0; j + 4 <= N; j += 4) {
+    double2 v[4][2];
+    tmem_get<4>(addr + 8 * j, v);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) f(j + i, v[i]);
+  }
+  if (N % 4) {
+    constexpr int R = N % 4 ? N % 4 : 1;
+    double2 v[R][2];
+    tmem_get<R>(addr + 8 * (N - R), v);
+#pragma unroll
+    for (int i = 0; i < R; ++i) f(N - R + i, v[i]);
+  }
+}
+
+// ---------------------------------------------------------- Gauss-Jordan --
+template <class C>
+struct GJ {
+  alignas(16) double2 lam[2];          // the panel's scale, double-buffered by column parity
+  alignas(16) unsigned key[8][C::NW];  // each warp's pivot key of each panel column
+  int fail;                            // status of the panel's pivots
+  int newpos[C::NP];                   // position after the panel of each panel row
+  int cmapinv[C::NP];
+};
+
+// Pivot key of a candidate entry: top bits of max(|re|, |im|) with the row
+// index in the low KB bits, so the unsigned maximum over a column picks the
+// largest entry up to a relative 2^-14 (KB = 6; 2^-12 for 8), ties to the
+// lowest row.
+template <int KB>
+__device__ __forceinline__ unsigned pivot_key(double2 v, int r) {
+  constexpr unsigned M = (1u << KB) - 1u;
+  return (hi_word(v) & ~M) | (M - (unsigned)r);
+}
+
+// Inverse of the matrix held in m (leading n x n block, identity padding) by
+// blocked Gauss-Jordan elimination with partial pivoting, into the shared
+// matrix out; scr (SCR complex, may be out itself) is scratch, park the thread's
+// TMEM columns for C::PARK tiles.  Ends with the
+// block synchronised.
+//
+// Columns are processed in panels of 8.  The n x 8 panel is factored in shared
+// memory by the whole block with one barrier per column and no division: it is
+// kept as W = lambda P (P the textbook Gauss-Jordan panel, lambda a complex
+// scalar) and, with p the pivot and s a power of two bringing p near 1,
+//     new(r, c) = (p s) a' - (s b') m,   lambda <- lambda p s
+//     a' = 0 if r is the pivot row or c the pivot column, else W(r, c)
+//     b' = -lambda for the pivot row, else W(r, j)
+//     m  =  lambda for the pivot column, else W(pivot row, c)
+// (expanding W = lambda P gives the textbook update times the new lambda;
+// |p s| lies in [1, 2.83]).  Pivot search is looked ahead: the threads that
+// write column j+1 of the panel reduce its pivot keys (see pivot_key) over the
+// rows not yet used as pivots, one slot per warp, before the barrier; the key's
+// exponent bits give s.
+//
+// The matrix itself never moves: a thread keeps its elements in registers for
+// the whole inversion and only tracks the position of its rows.  It writes its
+// part of the panel's 8 columns to shared memory at those positions, and its
+// part of the pivot rows once they are known; the rank-8 update then
+// accumulates in place on the tensor path,
+//     row r, columns Q: [r not a pivot row] W(r, Q) + P(r, :) W(pivot rows, Q),
+//     row r, panel:     P(r, :),                      P = W / lambda.
+// The row order and the undone column interchanges (column c of the inverse is
+// column t_{n-1}(...t_0(c)) of the eliminated matrix, t_k = (k b_k), b_k the
+// position of the k-th pivot) are applied as the result is written.  Keeping
+// the matrix in registers instead of two shared buffers removes its reload and
+// rewrite in each of the n/8 updates and is what lets several points share an SM.
+// Returns kOk, kSingular (all candidates zero or below 2^-1022) or kNonFinite
+// identically in every thread.
+template <class C>
+__device__ __forceinline__ int gj_invert(Acc<C>& m, double2* scr, double2* out, int n, const Lane& L, GJ<C>& sh,
+                                         uint32_t park = 0) {
+  constexpr int PE = C::PE, NP = C::NP, NW = C::NW;
+  constexpr int LPR = C::LPR, EPT = C::EPT, PS = C::PS;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const bool work = C::NW == C::WW || warp < C::WW;              // the warp has panel rows
+  const bool live = C::NTH == NP * LPR || tid < NP * LPR;        // the thread has one
+  const int pr_own = live ? tid / LPR : 0, cl = tid % LPR;
+  const int prow = pr_own * PS;
+  double2* const Bp = scr + 2 * PE;  // the panel's pivot rows [8][NP]
+  int pos[C::TR];  // position of each of the thread's matrix rows
+#pragma unroll
+  for (int i = 0; i < C::TR; ++i) pos[i] = L.r0 + 8 * i;
+  // The last warp (without panel rows where the block has warps to spare)
+  // keeps lambda and the permutations: lane l those of rows and columns l,
+  // l + 32, ...
+  const bool bk = warp == NW - 1;
+  constexpr bool kSpare = NW > C::WW;
+  constexpr bool kAll = NW <= C::WW + 1;  // every warp takes part in the pivot steps
+  constexpr unsigned kRow = (1u << C::KB) - 1u;
+  constexpr int RL = (NP + 31) / 32;
+  int cm[RL];  // t_k(...t_0(c)) over the steps done so far
+#pragma unroll
+  for (int i = 0; i < RL; ++i) cm[i] = lane + 32 * i;
+
+#pragma unroll 1
+  for (int k0 = 0, par = 0; k0 < n; k0 += 8, par ^= 1) {
+    const int jmax = (n - k0) < 8 ? (n - k0) : 8;
+    // A full panel's 8 steps end in the buffer they began in, so the next
+    // panel starts in the other one while this one may still be read.
+    double2* const P0 = scr + par * PE;
+    double2* const P1 = scr + (par ^ 1) * PE;
+    const int pj = (k0 - L.C0) >> 3;  // the panel's tile column among the thread's, if in range
+    // ---- publish the panel, keys of panel column 0 ----
+    unsigned key0 = 0u;
+#pragma unroll
+    for (int j = 0; j < C::TC; ++j)
+      if (j == pj) {
+#pragma unroll
+        for (int i = 0; i < C::TR; ++i) {
+          double2* row = P0 + pos[i] * PS + 2 * L.t;
+          row[0] = m.get(i, j, 0);
+          row[1] = m.get(i, j, 1);
+          if (L.t == 0 && pos[i] >= k0 && pos[i] < n) key0 = max(key0, pivot_key<C::KB>(m.get(i, j, 0), pos[i]));
+        }
+      }
+    key0 = __reduce_max_sync(0xffffffffu, key0);
+    if (lane == 0) sh.key[0][warp] = key0;
+    if (tid == 0) sh.lam[0] = make_double2(1.0, 0.0);
+    __syncthreads();
+    if (C::PARK) {
+#pragma unroll
+      for (int j = 0; j < C::PARK; ++j) {
+        const int jj = C::TC - C::PARK + j;
+        const double2 v[2] = {m.get(0, jj, 0), m.get(0, jj, 1)};
+        tmem_put(park + 8 * j, v);
+      }
+      tmem_stored();
+    }
+    // ---- factor the panel, one barrier per column, by the warps with panel
+    // rows and the bookkeeping warp; the others wait for the panel ----
+    if (work || bk) {
+      double2 av[EPT];  // this thread's panel elements
+#pragma unroll
+      for (int q = 0; q < EPT; ++q) av[q] = P0[prow + cl + LPR * q];
+      bool cand = live && pr_own >= k0 && pr_own < n;  // row not yet a pivot
+      int fail = kOk;  // the first bad pivot's status
+      int lg[RL];                                      // position of panel rows lane + 32 i
+#pragma unroll
+      for (int i = 0; i < RL; ++i) lg[i] = lane + 32 * i;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        if (j >= jmax) break;
+        const double2* Pc = (j & 1) ? P1 : P0;
+        double2* Pn = (j & 1) ? P0 : P1;
+        // What does not depend on the pivot is loaded with the key (one slot per
+        // warp; after the panel's first column only warps with rows post one).
+        const double2 fv = Pc[prow + j];
+        const double2 lam = sh.lam[j & 1];
+        unsigned key;
+        if (NW == 4) {
+          const uint4 kv = *reinterpret_cast<const uint4*>(sh.key[j]);
+          key = max(max(kv.x, kv.y), max(kv.z, kv.w));
+        } else if (NW == 2) {
+          const uint2 kv = *reinterpret_cast<const uint2*>(sh.key[j]);
+          key = max(kv.x, kv.y);
+        } else if (NW == 1) {
+          key = sh.key[j][0];
+        } else {
+          key = __reduce_max_sync(0xffffffffu, lane < (j == 0 ? NW : C::WW) ? sh.key[j][lane] : 0u);
+        }
+        // A zero or non-finite pivot ends the inversion at the end of the panel
+        // (off the path to the pivot row); min keeps its row in the panel.
+        const bool stop = key - (kRow + 1u) >= 0x7ff00000u - (kRow + 1u);
+        const int pr = min((int)(kRow - (key & kRow)), NP - 1);
+        const int ex = (int)(key >> 20);
+        const double sc = (ex != 0 && ex < 2046) ? __hiloint2double((2046 - ex) << 20, 0) : 1.0;
+        const double2* prow_p = Pc + pr * PS;
+        const double2 piv = prow_p[j];
+        const double2 ps = make_double2(piv.x * sc, piv.y * sc);
+        unsigned nk = 0u;
+        if (work) {
+          double2 mv[EPT];
+#pragma unroll
+          for (int q = 0; q < EPT; ++q) mv[q] = prow_p[cl + LPR * q];
+          const bool isp = pr_own == pr;
+          cand = cand && !isp;
+          const double2 bb = isp ? lam : fv;
+          const double nsc = isp ? sc : -sc;
+          const double2 nb = make_double2(bb.x * nsc, bb.y * nsc);  // -s b', so that nothing is negated below
+          const double2 pe = isp ? make_double2(0.0, 0.0) : ps;  // no branch: a' = 0 as a zero factor
+          // The next pivot column first, so that its keys are reduced under the
+          // other columns' updates.
+#pragma unroll
+          for (int qq = 0; qq < EPT; ++qq) {
+            const int q = (qq + (j + 1) / LPR) % EPT;
+            const int c = cl + LPR * q;
+            const bool pivcol = q == j / LPR && cl == j % LPR;
+            const double2 mq = pivcol ? lam : mv[q];
+            double2 v = make_double2(fma(nb.x, mq.x, -nb.y * mq.y), fma(nb.x, mq.y, nb.y * mq.x));
+            cfma(v, pivcol ? make_double2(0.0, 0.0) : pe, av[q]);
+            if (live) Pn[prow + c] = v;
+            av[q] = v;
+            if (j + 1 < 8 && qq == 0) {
+              if (cl == (j + 1) % LPR && cand) nk = pivot_key<C::KB>(v, pr_own);
+              nk = __reduce_max_sync(0xffffffffu, nk);
+            }
+          }
+        }
+        if (j + 1 < 8 && lane == 0) sh.key[j + 1][warp] = nk;
+        if (bk) {
+          double2 ln = cmul(lam, ps);
+          if (kSpare && j == 7) ln = crecip_smith(ln);  // under the other warps' element updates
+          if (lane == 0) sh.lam[(j + 1) & 1] = ln;
+          // the row interchange of this step: positions k and bl
+          const int k = k0 + j;
+          int x = lg[0];
+#pragma unroll
+          for (int i = 1; i < RL; ++i) x = (pr >> 5) == i ? lg[i] : x;
+          const int bl = __shfl_sync(0xffffffffu, x, pr & 31);
+#pragma unroll
+          for (int i = 0; i < RL; ++i) {
+            lg[i] = lane + 32 * i == pr ? k : (lg[i] == k ? bl : lg[i]);
+            cm[i] = cm[i] == k ? bl : (cm[i] == bl ? k : cm[i]);
+            if (j + 1 == jmax && lane + 32 * i < NP) sh.newpos[lane + 32 * i] = lg[i];
+          }
+        }
+        if (stop) fail = fail ? fail : (key <= kRow ? kSingular : kNonFinite);
+        if (j + 1 < jmax) {
+          if (kAll) __syncthreads();
+          else asm volatile("bar.sync 1, %0;" ::"n"(32 * (C::WW + 1)) : "memory");
+        }
+      }
+      if (bk && lane == 0) sh.fail = fail;
+    }
+    __syncthreads();
+    // ---- rank-8 update in registers ----
+    if (sh.fail) return sh.fail;
+    if (C::PARK) {
+      double2 v[C::PARK ? C::PARK : 1][2];
+      tmem_get<C::PARK ? C::PARK : 1>(park, v);
+#pragma unroll
+      for (int j = 0; j < C::PARK; ++j)
+#pragma unroll
+        for (int q = 0; q < 2; ++q) m.set(0, C::TC - C::PARK + j, q, v[j][q]);
+    }
+    // The owners of the pivot rows hand out their elements before the panel.
+    int np[C::TR];
+#pragma unroll
+    for (int i = 0; i < C::TR; ++i) np[i] = sh.newpos[pos[i]];
+#pragma unroll
+    for (int i = 0; i < C::TR; ++i) {
+      if ((unsigned)(np[i] - k0) < (unsigned)jmax) {
+        double2* row = Bp + (np[i] - k0) * NP;
+        const int sw = swz(np[i]);
+#pragma unroll
+        for (int j = 0; j < C::TC; ++j)
+#pragma unroll
+          for (int q = 0; q < 2; ++q) {
+            row[L.C0 + 8 * j + ((2 * L.t + q) ^ sw)] = m.get(i, j, q);
+            m.set(i, j, q, make_double2(0.0, 0.0));
+          }
+      }
+    }
+    const double2* P = (jmax & 1) ? P1 : P0;
+    const double2 ll = sh.lam[jmax & 1];
+    const double2 il = kSpare && jmax == 8 ? ll : crecip_smith(ll);
+    AFrag a[C::TR];
+#pragma unroll
+    for (int i = 0; i < C::TR; ++i)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const double2 v = cmul(P[pos[i] * PS + L.t + 4 * h], il);
+        a[i].re[h] = v.x;
+        a[i].im[h] = v.y;
+      }
+    __syncthreads();
+    auto pivots = [&](AFrag& b, int j) {  // column tile j of the pivot rows
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int kk = L.t + 4 * h;
+        const double2 v = Bp[sidx<NP>(kk, L.C0 + 8 * j + L.g)];
+        b.re[h] = kk < jmax ? v.x : 0.0;
+        b.im[h] = kk < jmax ? v.y : 0.0;
+      }
+    };
+    AFrag b, bn;
+    pivots(b, 0);
+#pragma unroll
+    for (int j = 0; j < C::TC; ++j) {
+      if (j + 1 < C::TC) pivots(bn, j + 1);
+      if (j == pj) {  // the panel's columns take P(r, :) (warp-uniform)
+#pragma unroll
+        for (int i = 0; i < C::TR; ++i)
+#pragma unroll
+          for (int q = 0; q < 2; ++q) m.set(i, j, q, cmul(P[pos[i] * PS + 2 * L.t + q], il));
+      } else {
+#pragma unroll
+        for (int i = 0; i < C::TR; ++i) chunk(m.re[i][j], m.im[i][j], a[i], b);
+      }
+      b = bn;
+    }
+#pragma unroll
+    for (int i = 0; i < C::TR; ++i) pos[i] = np[i];
+  }
+  if (bk)
+#pragma unroll
+    for (int i = 0; i < RL; ++i)
+      if (lane + 32 * i < NP) sh.cmapinv[cm[i]] = lane + 32 * i;
+  __syncthreads();  // the last panel and its pivot rows are read, cmapinv is complete
+#pragma unroll
+  for (int j = 0; j < C::TC; ++j)
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int c = sh.cmapinv[L.c0 + 8 * j + q];
+#pragma unroll
+      for (int i = 0; i < C::TR; ++i) out[sidx<NP>(pos[i], c)] = m.get(i, j, q);
+    }
+  __syncthreads();
+  return kOk;
 }
 
 // Shared memory of a point: alpha, beta (or g, G0) and the third buffer, the

@@ -1,6 +1,7 @@
 """The one-point-per-block FP64 kernels at the edges of their tile splits.
 
-Orders just below, at and above each padded order (8, 16, 24, 32, 48), leads
+Orders just below, at and above each padded order (8, 16, 24, 32, 48, then
+every multiple of 8 up to 104, where the workspace kernels take over), leads
 of another order than the device, layers with their own blocks, and both tile
 splits of order 9..16 (chosen by the number of points).  Random systems at an
 eta that keeps the decimation well conditioned, against the CPU oracle to the
@@ -53,7 +54,9 @@ def _solve(s, omegas):
 @pytest.mark.parametrize("n,nl,nr,layers", [
     (2, 2, 2, 3), (7, 8, 7, 1), (8, 8, 3, 4), (9, 9, 9, 2), (15, 16, 2, 3), (16, 16, 16, 3), (17, 17, 9, 2),
     (23, 24, 23, 3), (24, 24, 24, 1), (25, 25, 8, 2), (31, 32, 31, 2), (32, 32, 32, 3), (33, 33, 25, 2),
-    (40, 40, 41, 2), (47, 48, 47, 3), (48, 48, 48, 2), (5, 48, 20, 2)])
+    (40, 40, 41, 2), (47, 48, 47, 3), (48, 48, 48, 2), (5, 48, 20, 2), (49, 49, 48, 2), (56, 57, 56, 1),
+    (64, 64, 10, 3), (65, 65, 64, 2), (72, 72, 72, 2), (73, 80, 73, 2), (81, 88, 50, 1), (89, 96, 89, 2),
+    (96, 96, 96, 3), (97, 104, 97, 2), (104, 104, 104, 2), (105, 105, 104, 2), (20, 104, 60, 3)])
 def test_orders_match_oracle(n, nl, nr, layers):
     s = _system(n, nl, nr, layers, seed=100 * n + nl)
     omegas = np.array([0.3, 1.1, 1.9])
