@@ -42,7 +42,7 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     objdir = PKG / "_build"
     objdir.mkdir(exist_ok=True)
     flags = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-I", str(INCLUDE),
-                    "--expt-relaxed-constexpr"]
+                    "--expt-relaxed-constexpr", "-split-compile=0"]  # one optimiser thread per kernel instance
     objs = []
     procs = []
     for src in sources():

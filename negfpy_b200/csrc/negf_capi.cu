@@ -392,7 +392,7 @@ size_t negf_device_green_workspace_bytes(int n_dev, int n_lead_l, int n_lead_r, 
   if (n_dev <= 0 || n_lead_l <= 0 || n_lead_r <= 0 || n_layers <= 0) return 0;
   const int nmax = max3(n_dev, n_lead_l, n_lead_r);
   if (nmax > 256) return 0;
-  const int np = (nmax + 15) / 16 * 16;
+  const int np = negf::adj_order(nmax);
   const int grid = negf::full_grid(np);
   if (grid <= 0) return 0;
   return kCounterBytes + negf::full_ws_bytes(np, n_dev, n_layers, grid);
@@ -417,7 +417,7 @@ int negf_device_green_f64(int n_dev, int n_lead_l, int n_lead_r, int n_layers, i
     return fail(NEGF_EINVAL, "negf_device_green_f64: negative stride");
   const int nmax = max3(n_dev, n_lead_l, n_lead_r);
   if (nmax > 256) return fail(NEGF_EUNSUPPORTED, "negf_device_green_f64: block order above 256");
-  const int np = (nmax + 15) / 16 * 16;
+  const int np = negf::adj_order(nmax);
   const int grid = negf::full_grid(np);
   if (grid <= 0) return cuda_fail("negf_device_green_f64: occupancy query");
   if (!workspace || workspace_bytes < kCounterBytes + negf::full_ws_bytes(np, n_dev, n_layers, grid))
@@ -468,7 +468,7 @@ size_t negf_adjoint_workspace_bytes(int n_dev, int n_lead_l, int n_lead_r, int n
   if (n_dev <= 0 || n_lead_l <= 0 || n_lead_r <= 0 || n_layers <= 0) return 0;
   const int nmax = max3(n_dev, n_lead_l, n_lead_r);
   if (nmax > 256) return 0;
-  const int np = (nmax + 15) / 16 * 16;
+  const int np = negf::adj_order(nmax);
   const int grid = negf::grad_grid(np);
   if (grid <= 0) return 0;
   return kCounterBytes + negf::grad_ws_bytes(np, n_dev, n_layers, grid);
@@ -509,7 +509,7 @@ static int rgf_adjoint_common(const char* name, int n_dev, int n_lead_l, int n_l
     return fail2(NEGF_EINVAL, name, "negative stride");
   const int nmax = max3(n_dev, n_lead_l, n_lead_r);
   if (nmax > 256) return fail2(NEGF_EUNSUPPORTED, name, "block order above 256");
-  const int np = (nmax + 15) / 16 * 16;
+  const int np = negf::adj_order(nmax);
   const int grid = negf::grad_grid(np);
   if (grid <= 0) return cuda_fail2(name, "occupancy query");
   if (!workspace || workspace_bytes < kCounterBytes + negf::grad_ws_bytes(np, n_dev, n_layers, grid))
@@ -617,7 +617,7 @@ int negf_rgf_adjoint_points_f64(int n_dev, int n_lead_l, int n_lead_r, int n_lay
 
 size_t negf_sgf_adjoint_workspace_bytes(int n_lead, int n_dev) {
   if (n_lead <= 0 || n_dev <= 0 || n_lead > 256 || n_dev > 256) return 0;
-  const int np = (max3(n_lead, n_dev, 1) + 15) / 16 * 16;
+  const int np = negf::adj_order(max3(n_lead, n_dev, 1));
   const int grid = negf::sgf_adj_grid(np);
   if (grid <= 0) return 0;
   return kCounterBytes + negf::sgf_adj_ws_bytes(np, grid);
@@ -638,7 +638,7 @@ static int sgf_adjoint_common(const char* name, int per_point, int n_lead, int n
     return fail2(NEGF_EINVAL, name, "negative stride");
   if (maxiter <= 0 || !(tol > 0.0)) return fail2(NEGF_EINVAL, name, "maxiter and tol must be positive");
   if (n_lead > 256 || n_dev > 256) return fail2(NEGF_EUNSUPPORTED, name, "block order above 256");
-  const int np = (max3(n_lead, n_dev, 1) + 15) / 16 * 16;
+  const int np = negf::adj_order(max3(n_lead, n_dev, 1));
   const int grid = negf::sgf_adj_grid(np);
   if (grid <= 0) return cuda_fail2(name, "occupancy query");
   if (!workspace || workspace_bytes < kCounterBytes + negf::sgf_adj_ws_bytes(np, grid))

@@ -109,6 +109,15 @@ size_t sr_ws_bytes(int np, int grid);
 size_t rgf_ws_bytes(int np, int n, int grid);
 int sr_launch(const SrArgs& a, int np, int grid, double2* ws, unsigned* counter, cudaStream_t st);
 int rgf_launch(const RgfArgs& a, int np, int grid, double2* ws, cudaStream_t st);
+int grad_grid(int np);
+size_t grad_ws_bytes(int np, int n, int L, int grid);
+int grad_launch(const GradArgs& ga, int np, int grid, double2* ws, cudaStream_t st);
+int sgf_adj_grid(int np);
+size_t sgf_adj_ws_bytes(int np, int grid);
+int sgf_adj_launch(const SgfAdjArgs& sa, int np, int grid, double2* ws, cudaStream_t st);
+int full_grid(int np);
+size_t full_ws_bytes(int np, int n, int L, int grid);
+int full_launch(const FullArgs& fa, int np, int grid, double2* ws, cudaStream_t st);
 }  // namespace mid
 // Block orders 49..256 (those above 104 padded to a multiple of 16): global-memory workspace.
 int global_order(int n);  // padded order for n > 48, 0 if unsupported
@@ -148,6 +157,8 @@ int batch_launch(const ::NegfBatchSystem* sys, int n_systems, const int* item_sy
                  const double* item_omega, int n_items, double tol, int maxiter, double* t_out, int* status_out,
                  int* iters_out, int npmax, int mixed, int minb, int grid, void* counter, void* ws, cudaStream_t st);
 
+// Adjoints and full G: np = adj_order(largest order), 0 if unsupported.
+int adj_order(int n);
 size_t full_ws_bytes(int np, int n, int L, int grid);
 int full_grid(int np);
 int full_f64_launch(const FullArgs& fa, int np, int grid, double2* ws, cudaStream_t st);

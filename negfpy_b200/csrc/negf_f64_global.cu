@@ -1,5 +1,5 @@
 // FP64 kernels for block orders 105..256 (padded to NP, a multiple of 16), and
-// the adjoint and full-G kernels of every order up to 256.
+// the adjoint and full-G kernels of these orders.
 //
 // Beyond n = 104 a block's registers do not hold a matrix, so here all of them
 // live in a per-block workspace in global memory (mostly L2 resident) and the
@@ -726,9 +726,11 @@ int sr_f64_global_launch(const SrArgs& a, int np, int grid, double2* ws, unsigne
 }
 
 size_t grad_ws_bytes(int np, int n, int L, int grid) {
+  if (np <= mid::kMaxOrder) return mid::grad_ws_bytes(np, n, L, grid);
   return (size_t)grid * ((14 + 2 * (size_t)L) * np * np + 2 * (size_t)n * n) * 16;
 }
 int grad_grid(int np) {
+  if (np <= mid::kMaxOrder) return mid::grad_grid(np);
   const int g = glob::occupancy_grid(glob::rgf_grad_f64_kernel, np);
   int dev = 0, nsm = 0;
   cudaGetDevice(&dev);
@@ -736,9 +738,11 @@ int grad_grid(int np) {
   return g > 2 * nsm ? 2 * nsm : g;  // two blocks per SM bound the 2L-slot workspace
 }
 size_t full_ws_bytes(int np, int n, int L, int grid) {
+  if (np <= mid::kMaxOrder) return mid::full_ws_bytes(np, n, L, grid);
   return (size_t)grid * ((6 + 3 * (size_t)L) * np * np + 2 * (size_t)n * n) * 16;
 }
 int full_grid(int np) {
+  if (np <= mid::kMaxOrder) return mid::full_grid(np);
   const int g = glob::occupancy_grid(glob::rgf_full_f64_kernel, np);
   int dev = 0, nsm = 0;
   cudaGetDevice(&dev);
@@ -747,11 +751,16 @@ int full_grid(int np) {
 }
 int full_f64_launch(const FullArgs& fa, int np, int grid, double2* ws, cudaStream_t st) {
   if (fa.r.batch <= 0) return 0;
+  if (np <= mid::kMaxOrder) return mid::full_launch(fa, np, grid, ws, st);
   glob::rgf_full_f64_kernel<<<grid, glob::kThreads, glob::smem_bytes(np), st>>>(fa, np, ws);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
-size_t sgf_adj_ws_bytes(int np, int grid) { return (size_t)grid * 15 * (size_t)np * np * 16; }
+size_t sgf_adj_ws_bytes(int np, int grid) {
+  if (np <= mid::kMaxOrder) return mid::sgf_adj_ws_bytes(np, grid);
+  return (size_t)grid * 15 * (size_t)np * np * 16;
+}
 int sgf_adj_grid(int np) {
+  if (np <= mid::kMaxOrder) return mid::sgf_adj_grid(np);
   const int g = glob::occupancy_grid(glob::sgf_adjoint_f64_kernel, np);
   int dev = 0, nsm = 0;
   cudaGetDevice(&dev);
@@ -760,11 +769,13 @@ int sgf_adj_grid(int np) {
 }
 int sgf_adj_launch(const SgfAdjArgs& sa, int np, int grid, double2* ws, cudaStream_t st) {
   if (sa.batch <= 0) return 0;
+  if (np <= mid::kMaxOrder) return mid::sgf_adj_launch(sa, np, grid, ws, st);
   glob::sgf_adjoint_f64_kernel<<<grid, glob::kThreads, glob::smem_bytes(np), st>>>(sa, np, ws);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 int grad_f64_launch(const GradArgs& ga, int np, int grid, double2* ws, cudaStream_t st) {
   if (ga.r.batch <= 0) return 0;
+  if (np <= mid::kMaxOrder) return mid::grad_launch(ga, np, grid, ws, st);
   glob::rgf_grad_f64_kernel<<<grid, glob::kThreads, glob::smem_bytes(np), st>>>(ga, np, ws);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
@@ -779,6 +790,12 @@ int rgf_f64_global_launch(const RgfArgs& a, int np, int grid, double2* ws, cudaS
 }  // namespace negf
 
 namespace negf {
+int adj_order(int n) {
+  if (n <= 0 || n > 256) return 0;
+  for (int np : {16, 24, 32, 48, 64, 72, 80, 96, 104})
+    if (n <= np) return np;
+  return (n + 15) / 16 * 16;
+}
 int global_order(int n) {
   if (n <= 48 || n > 256) return 0;
   return n <= mid::kMaxOrder ? (n + 7) / 8 * 8 : (n + 15) / 16 * 16;

@@ -9,38 +9,12 @@
 // second block does not fit.  Parking tiles takes the pivot steps of the
 // decimation from 745 to 600 cycles at n = 96 (spills); the device solve does
 // not gain from it.
-#include <atomic>
-
-#include "negf_mid.cuh"
+#include "negf_mid_launch.cuh"
 
 namespace negf {
 namespace mid {
 
-template <class C>
-static int grid_of() {
-  static std::atomic<int> sms[64];
-  int dev = 0;
-  cudaGetDevice(&dev);
-  int n = dev < 64 ? sms[dev].load(std::memory_order_acquire) : 0;
-  if (n == 0) {
-    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return -3;
-    if (dev < 64) sms[dev].store(n, std::memory_order_release);
-  }
-  return n * C::OCC;
-}
-template <class C, class K>
-static int raise_smem(K kernel) {
-  static std::atomic<bool> done[64];
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 64 && done[dev].load(std::memory_order_acquire)) return 0;
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared_bytes<C>()) != cudaSuccess)
-    return -3;
-  if (dev < 64) done[dev].store(true, std::memory_order_release);
-  return 0;
-}
-
-// f with the split of the padded order, -2 for another order.
+// f with the split of the padded order (56 .. 104).
 template <class F>
 static auto with_sr(int np, F&& f) {
   switch (np) {
@@ -82,7 +56,7 @@ int sr_launch(const SrArgs& a, int np, int grid, double2* ws, unsigned* counter,
   if (a.batch <= 0) return 0;
   return with_sr(np, [&](auto c) {
     using C = decltype(c);
-    if (raise_smem<C>(sr_kernel<C>)) return -3;
+    if (raise_smem<sr_kernel<C>, C>()) return -3;
     sr_kernel<C><<<grid < a.batch ? grid : a.batch, C::NTH, shared_bytes<C>(), st>>>(a, ws, counter);
     return cudaGetLastError() == cudaSuccess ? 0 : -3;
   });
@@ -91,7 +65,7 @@ int rgf_launch(const RgfArgs& a, int np, int grid, double2* ws, cudaStream_t st)
   if (a.batch <= 0) return 0;
   return with_rgf(np, [&](auto c) {
     using C = decltype(c);
-    if (raise_smem<C>(rgf_kernel<C>)) return -3;
+    if (raise_smem<rgf_kernel<C>, C>()) return -3;
     rgf_kernel<C><<<grid < a.batch ? grid : a.batch, C::NTH, shared_bytes<C>(), st>>>(a, ws);
     return cudaGetLastError() == cudaSuccess ? 0 : -3;
   });

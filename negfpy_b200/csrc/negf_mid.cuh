@@ -343,6 +343,13 @@ __device__ __forceinline__ void self_energy(double2* S, const double2* V, const 
   __syncthreads();
 }
 
+// Element of Gamma = i (Sigma - Sigma^H), zero outside n x n.
+__device__ __forceinline__ double2 gamma_of(const double2* S, int n, int r, int c) {
+  if (r >= n || c >= n) return make_double2(0.0, 0.0);
+  const double2 d = csub(S[r * n + c], cconj(S[c * n + r]));
+  return make_double2(-d.y, d.x);
+}
+
 // T = Re sum_ij (Gamma_L G Gamma_R)_ij conj(G)_ij for G in the row-major
 // workspace; GL, U: workspace.  The terms are summed as 8 warps walking 16 x 16
 // tiles of the largest order nmax would (an order that does not depend on the
@@ -353,13 +360,8 @@ __device__ __forceinline__ double trace_t(const double2* sigL, const double2* si
                                           double2* U, int n, int nmax, double2* X, double* red, const Lane& L) {
   constexpr int NP = C::NP;
   const int tid = threadIdx.x, kch = (n + 7) >> 3;
-  auto gamma = [&](const double2* S, int r, int cc) {
-    if (r >= n || cc >= n) return make_double2(0.0, 0.0);
-    const double2 d = csub(S[r * n + cc], cconj(S[cc * n + r]));
-    return make_double2(-d.y, d.x);
-  };
   Acc<C> c;
-  tiles<C>(L, [&](int, int, int r, int cc) { GL[r * NP + cc] = gamma(sigL, r, cc); });
+  tiles<C>(L, [&](int, int, int r, int cc) { GL[r * NP + cc] = gamma_of(sigL, n, r, cc); });
   __syncwarp();
   load_x<C>(X, G, NP, NP, NP);
   __syncthreads();
@@ -367,7 +369,7 @@ __device__ __forceinline__ double trace_t(const double2* sigL, const double2* si
   prod<C, false, false>(c, gl, X, kch, L);
   store_rows<C>(U, c, L);
   __syncthreads();
-  tiles<C>(L, [&](int, int, int r, int cc) { X[sidx<NP>(r, cc)] = gamma(sigR, r, cc); });
+  tiles<C>(L, [&](int, int, int r, int cc) { X[sidx<NP>(r, cc)] = gamma_of(sigR, n, r, cc); });
   __syncthreads();
   prod<C, false, false>(c, u, X, kch, L);
   __syncthreads();

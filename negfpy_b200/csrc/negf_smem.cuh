@@ -457,10 +457,10 @@ __device__ __forceinline__ int gj_invert(Acc<C>& m, double2* scr, double2* out, 
         const double2 fv = Pc[prow + j];
         const double2 lam = sh.lam[j & 1];
         unsigned key;
-        if (NW == 4) {
+        if (NW == 4 && kAll) {  // every slot is posted in every step
           const uint4 kv = *reinterpret_cast<const uint4*>(sh.key[j]);
           key = max(max(kv.x, kv.y), max(kv.z, kv.w));
-        } else if (NW == 2) {
+        } else if (NW == 2 && kAll) {
           const uint2 kv = *reinterpret_cast<const uint2*>(sh.key[j]);
           key = max(kv.x, kv.y);
         } else if (NW == 1) {

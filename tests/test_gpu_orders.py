@@ -81,3 +81,78 @@ def test_both_splits_of_order_16_agree_bitwise(n):
         gp, dp, tp, ip = _solve(s, omegas[a:b])
         for x, y in ((g, gp), (dos, dp), (t, tp), (it, ip)):
             assert np.array_equal(x[a:b], y)
+
+
+def _dense(s, z, sl, sr):
+    """A of the device as a torch complex128 matrix (differentiable in the blocks)."""
+    n, layers = s["on"][0].shape[0], len(s["on"])
+    rows = []
+    for i in range(layers):
+        row = [torch.zeros((n, n), dtype=torch.complex128) for _ in range(layers)]
+        row[i] = z * torch.eye(n, dtype=torch.complex128) - s["on"][i]
+        if i == 0:
+            row[i] = row[i] - sl
+        if i == layers - 1:
+            row[i] = row[i] - sr
+        if i + 1 < layers:
+            row[i + 1] = -s["cp"][i]
+        if i > 0:
+            row[i - 1] = -s["cp"][i - 1].mH
+        rows.append(torch.cat(row, 1))
+    return torch.cat(rows, 0)
+
+
+@pytest.mark.parametrize("n,nl,nr,layers", [
+    (3, 3, 3, 2), (16, 16, 9, 1), (17, 24, 17, 3), (25, 25, 25, 2), (33, 48, 33, 2), (49, 49, 64, 2), (65, 65, 72, 3),
+    (73, 73, 80, 2), (81, 96, 81, 2), (97, 97, 104, 2), (105, 105, 105, 2)])
+def test_adjoint_and_full_green_orders(n, nl, nr, layers):
+    """The adjoint blocks, self-energy adjoints, surface-GF adjoint and full G at
+    the edges of their padded orders, against torch autograd through the dense
+    device matrix (1e-10 of the largest entry: the solves are well conditioned
+    at this eta)."""
+    s = _system(n, nl, nr, layers, seed=7 * n + layers)
+    w, z = 1.1, (1.1 + 1j * ETA) ** 2
+    c = lambda x: torch.as_tensor(x[None], device="cuda").contiguous()  # noqa: E731
+    om = torch.tensor([w], dtype=torch.float64, device="cuda")
+    eta = torch.full_like(om, ETA)
+    ki = torch.zeros(1, dtype=torch.int32, device="cuda")
+    rl = engine.sgf_sr(c(s["l"][0]), c(s["l"][1]), None, om, eta, ki)
+    rr = engine.sgf_sr(c(s["r"][0]), c(s["r"][1]), None, om, eta, ki)
+    on = c(np.stack(s["on"]))
+    cp = c(np.stack(s["cp"])) if layers > 1 else None
+    vl, vr = c(s["vl"]), c(s["vr"])
+    wt = torch.ones(1, dtype=torch.float64, device="cuda")
+    t, st, x_on, x_cp, xs_l, xs_r = engine.rgf_adjoint(on, cp, layers, vl, vr, rl["g"], rr["g"], om, eta, ki, None, wt,
+                                                       want_sigma=True, deterministic=True)
+    gg, gsl, gsr, gst = engine.device_green(on, cp, layers, vl, vr, rl["g"], rr["g"], om, eta, ki, None)
+    ad = engine.sgf_adjoint(c(s["l"][1]), None, vl, rl["g"], xs_l, ki, deterministic=True)
+    assert int(st[0]) == 0 and int(gst[0]) == 0 and int(ad["status"][0]) == 0
+    # reference: leaves are the blocks, V_L, V_R and both surface GFs
+    lf = lambda x: torch.as_tensor(x).clone().requires_grad_(True)  # noqa: E731
+    ref = {"on": [lf(b) for b in s["on"]], "cp": [lf(b) for b in s["cp"]]}
+    tvl, tvr = lf(s["vl"]), lf(s["vr"])
+    tg = [lf(r["g"][0].cpu().numpy()) for r in (rl, rr)]
+    sl, sr = tvl @ tg[0] @ tvl.mH, tvr @ tg[1] @ tvr.mH
+    sl.retain_grad(), sr.retain_grad()
+    g = torch.linalg.inv(_dense(ref, z, sl, sr))
+    g0 = g[:n, (layers - 1) * n:]
+    tt = torch.trace(1j * (sl - sl.mH) @ g0 @ (1j * (sr - sr.mH)) @ g0.mH).real
+    tt.backward()
+    near = lambda a, b: float((a - b).abs().max()) <= TOL * float(b.abs().max())  # noqa: E731
+    adj = lambda x: 2.0 * x.cpu().conj().transpose(-1, -2)  # noqa: E731  (torch's gradient from X)
+    assert abs(t[0].item() - tt.item()) <= TOL * max(1.0, abs(tt.item()))
+    assert near(gg[0].cpu(), g.detach()) and near(gsl[0].cpu(), sl.detach()) and near(gsr[0].cpu(), sr.detach())
+    assert near(adj(x_on[0]), torch.stack([b.grad for b in ref["on"]]))
+    if layers > 1:
+        assert near(adj(x_cp[0]), torch.stack([b.grad for b in ref["cp"]]))
+    assert near(adj(xs_l[0]), sl.grad) and near(adj(xs_r[0]), sr.grad)
+    assert near(adj(ad["v"][0]), tvl.grad)
+    # H00bar = g Lam g with Lam - Q Lam P = gbar, P = g H01, Q = H01^H g, gbar = V^H X V
+    gl, h01 = rl["g"][0].cpu(), torch.as_tensor(s["l"][1])
+    v, x = tvl.detach(), xs_l[0].cpu()
+    lam, a, b = v.mH @ x @ v, h01.mH @ gl, gl @ h01
+    for _ in range(60):
+        lam, a, b = lam + a @ lam @ b, a @ a, b @ b
+    h00 = gl @ lam @ gl
+    assert near(ad["h00"][0].cpu(), h00)
+    assert near(ad["h01"][0].cpu(), gl @ h01.mH @ h00 + (h00 @ h01 @ gl).mH)
