@@ -31,13 +31,17 @@ def _stack_leads(lead, kpoints):
 
 
 def _dos_batch(omegas, lead, kpoints, etas, normalize_per_mode):
-    """DOS and status for points (omega_i, k_i, eta_i), one launch."""
+    """DOS and status for points (omega_i, k_i, eta_i), one launch.  With fewer
+    ``kpoints`` than ``omegas`` the points run over them in turn (omega-major):
+    every k is resolved and uploaded once, whatever the number of omegas."""
     dev = _lib.require_cuda()
     d00, d01, d10 = _stack_leads(lead, kpoints)
-    P = len(kpoints)
+    K, P = len(kpoints), len(omegas)
     om = torch.tensor(np.asarray(omegas, dtype=float), dtype=torch.float64, device=dev)
     et = torch.tensor(np.asarray(etas, dtype=float), dtype=torch.float64, device=dev)
-    ki = torch.arange(P, dtype=torch.int32, device=dev)
+    ki = torch.arange(K, dtype=torch.int32, device=dev)
+    if P != K:
+        ki = ki.repeat(P // K)
     r = engine.sgf_sr(engine._c(d00), engine._c(d01), None if d10 is None else engine._c(d10), om, et, ki,
                       want_g=False, want_dos=True)
     dos = r["dos"].cpu().numpy()
@@ -138,9 +142,8 @@ def lead_surface_dos_spectrum(omegas: Iterable[float], lead, *, kpoints: list | 
     ks = [None] if kpoints is None else list(kpoints)
     K = len(ks)
     om = np.repeat(omega_arr, K)
-    kk = ks * omega_arr.size
-    d, st = _dos_batch(om, lead, kk, [eta] * om.size, normalize_per_mode)
-    for s in st:
+    d, st = _dos_batch(om, lead, ks, np.full(om.size, eta), normalize_per_mode)
+    for s in st[st != _lib.OK]:
         raise_for_status(int(s))
     return d.reshape(omega_arr.size, K).mean(axis=1)
 

@@ -39,6 +39,20 @@ def _r(t, device=None) -> torch.Tensor:
     return t.to(device=device or _dev(), dtype=RDT).contiguous()
 
 
+def _upload(arrays, device) -> list:
+    """``_c`` of several host arrays (None stays None): small ones go to the
+    device in one copy and come back as views of it (each copy from pageable
+    memory costs about 10 us of host time)."""
+    host = [a if isinstance(a, torch.Tensor) or a is None else np.asarray(a) for a in arrays]
+    small = [i for i, a in enumerate(host) if isinstance(a, np.ndarray) and a.size <= 1 << 14]
+    out = [None if a is None else a if i in small else _c(a, device) for i, a in enumerate(host)]
+    if small:
+        flat = torch.from_numpy(np.concatenate([host[i].astype(np.complex128, copy=False).ravel() for i in small]))
+        for i, part in zip(small, flat.to(device).split([host[i].size for i in small])):
+            out[i] = part.view(host[i].shape)
+    return out
+
+
 def sgf_sr(d00: torch.Tensor, d01: torch.Tensor, d10: torch.Tensor | None, omega: torch.Tensor, eta: torch.Tensor,
            k_index: torch.Tensor | None = None, tol: float = 1e-12, maxiter: int = 200, want_g: bool = True,
            want_dos: bool = False, stream=None) -> dict:
@@ -508,14 +522,11 @@ class StackedSystem:
         matched-contact couplings V_L = d10 (or d01^H) and V_R = d01 (core/negf.py:192-201),
         contacting the whole first / last layer."""
         dev = _dev()
-        ll = (_c(lead_l["d00"], dev), _c(lead_l["d01"], dev),
-              None if lead_l.get("d10") is None else _c(lead_l["d10"], dev))
         if same_leads is None:
             same_leads = lead_r is lead_l
-        lr = ll if same_leads else (_c(lead_r["d00"], dev), _c(lead_r["d01"], dev),
-                                    None if lead_r.get("d10") is None else _c(lead_r["d10"], dev))
-        on = _c(onsite, dev)
-        cp = None if coupling is None else _c(coupling, dev)
+        *ll, on, cp, vl, vr = _upload([lead_l["d00"], lead_l["d01"], lead_l.get("d10"), onsite, coupling, vl, vr], dev)
+        ll = tuple(ll)
+        lr = ll if same_leads else tuple(_upload([lead_r["d00"], lead_r["d01"], lead_r.get("d10")], dev))
         n = on.shape[-1]
         if vl is None:
             vl = ll[2] if ll[2] is not None else ll[1].conj().transpose(-1, -2)
@@ -558,14 +569,16 @@ class StackedSystem:
         eta = _r(eta, dev)
         eta_dev = eta if eta_dev is None else _r(eta_dev, dev)
         k_index = k_index.to(device=dev, dtype=torch.int32).contiguous()
-        T = torch.empty(P, dtype=RDT, device=dev)
-        st = torch.empty(P, dtype=torch.int32, device=dev)
-        itl = torch.empty(P, dtype=torch.int32, device=dev)
-        itr = torch.empty(P, dtype=torch.int32, device=dev)
         if chunk is None:
             per_point = 16 * (self.nl * self.nl + (0 if self.same_leads else self.nr * self.nr))
             chunk = max(4096, (8 << 30) // per_point)
         chunk = max(1, int(chunk))
+        whole = 0 < P <= chunk  # one chunk: its results are the results
+        if not whole:
+            T = torch.empty(P, dtype=RDT, device=dev)
+            st = torch.empty(P, dtype=torch.int32, device=dev)
+            itl = torch.empty(P, dtype=torch.int32, device=dev)
+            itr = torch.empty(P, dtype=torch.int32, device=dev)
         for a in range(0, P, chunk):
             b = min(P, a + chunk)
             sl = slice(a, b)
@@ -589,6 +602,9 @@ class StackedSystem:
             else:
                 t, s = rgf_transmission(self.onsite, self.coupling, self.n_layers, self.vl, self.vr, rl["g"],
                                         rr["g"], om, ed, ki, lst, stream=stream)
+            if whole:
+                T, st, itl, itr = t, s, rl["iters"], rr["iters"] if rr is not rl else rl["iters"].clone()
+                break
             T[sl] = t
             st[sl] = s
             itl[sl] = rl["iters"]

@@ -171,7 +171,7 @@ def material_kspace_stack(params: MaterialKspaceParams, kpoints: list, layer_mas
             lm = np.repeat(np.asarray(params.masses, dtype=float)[None, :], n_layers, axis=0)
         else:
             lm = np.asarray(layer_masses, dtype=float)
-        ms = np.stack([_inv_sqrt_mass(lm[i], params.dof_per_atom) for i in range(n_layers)])  # [L, n]
+        ms = 1.0 / np.sqrt(np.repeat(lm, params.dof_per_atom, axis=1))  # [L, n]
         out["onsite"] = ms[None, :, :, None] * phi00[:, None] * ms[None, :, None, :]
         out["coupling"] = ms[None, :-1, :, None] * phi01[:, None] * ms[None, 1:, None, :]
     return out

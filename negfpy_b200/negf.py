@@ -70,7 +70,7 @@ def point_system(omega, device, lead_left, lead_right, eta, eta_device=None, kpa
     vdl_left = _resolve_coupling(device_to_lead_left, kpar)
     vdl_right = _resolve_coupling(device_to_lead_right, kpar)
     left = resolve_lead_blocks(lead_left, kpar)
-    right = resolve_lead_blocks(lead_right, kpar)
+    right = left if lead_right is lead_left else resolve_lead_blocks(lead_right, kpar)
     npl = dev.dof_per_layer
     L = dev.n_layers
     dim = L * npl
@@ -83,8 +83,9 @@ def point_system(omega, device, lead_left, lead_right, eta, eta_device=None, kpa
     coupling = [np.asarray(b, dtype=np.complex128) for b in dev.coupling_blocks]
     ll = [np.asarray(left.d00, dtype=np.complex128), np.asarray(left.d01, dtype=np.complex128),
           None if left.d10 is None else np.asarray(left.d10, dtype=np.complex128)]
-    lr = [np.asarray(right.d00, dtype=np.complex128), np.asarray(right.d01, dtype=np.complex128),
-          None if right.d10 is None else np.asarray(right.d10, dtype=np.complex128)]
+    lr = ll if right is left else [np.asarray(right.d00, dtype=np.complex128),
+                                   np.asarray(right.d01, dtype=np.complex128),
+                                   None if right.d10 is None else np.asarray(right.d10, dtype=np.complex128)]
     if omega_scale is not None:
         scale = float(omega_scale)
         if scale <= 0.0:
@@ -95,8 +96,9 @@ def point_system(omega, device, lead_left, lead_right, eta, eta_device=None, kpa
         eta_dev /= scale
         onsite = [_scaled(b, s2) for b in onsite]
         coupling = [_scaled(b, s2) for b in coupling]
+        shared = lr is ll
         ll = [None if b is None else _scaled(b, s2) for b in ll]
-        lr = [None if b is None else _scaled(b, s2) for b in lr]
+        lr = ll if shared else [None if b is None else _scaled(b, s2) for b in lr]
     if vdl_left is None:
         vdl_left = ll[2] if ll[2] is not None else ll[1].conj().T
     if vdl_right is None:
@@ -142,7 +144,7 @@ def _same_lead(a: list, b: list) -> bool:
     for x, y in zip(a, b):
         if (x is None) != (y is None):
             return False
-        if x is not None and (x.shape != y.shape or not np.array_equal(x, y)):
+        if x is not y and (x.shape != y.shape or not np.array_equal(x, y)):
             return False
     return True
 
@@ -301,6 +303,13 @@ def _classify(t, st, max_allowed, nonneg_tol):
     return None
 
 
+def _accepted(t, st, max_allowed, nonneg_tol):
+    """Boolean mask of the points ``_classify`` accepts."""
+    with np.errstate(invalid="ignore"):
+        ok = (st == _lib.OK) & np.isfinite(t) & ~(t < -float(nonneg_tol))
+        return ok if max_allowed is None else ok & ~(t > max_allowed)
+
+
 def _prepare_ladder_systems(omega, device, lead_left, lead_right, kpoints, eta_device, device_to_lead_left,
                             device_to_lead_right, contact_left_indices, contact_right_indices, omega_scale):
     systems = _systems_over_k(omega, device, lead_left, lead_right, kpoints, 1.0, eta_device, device_to_lead_left,
@@ -335,7 +344,7 @@ def transmission_kavg_adaptive(omega: float, device, lead_left, lead_right, kpoi
                  device_to_lead_right, contact_left_indices, contact_right_indices, omega_scale)
     K = len(kpoints)
     # one call shares the lead order over its k points (stack_systems checks it)
-    max_allowed = [None if max_channel_factor is None else float(max_channel_factor) * float(kb.sys.nl)] * K
+    max_allowed = None if max_channel_factor is None else float(max_channel_factor) * float(kb.sys.nl)
     accepted: dict[int, tuple[float, float]] = {}
     attempts: list[tuple[int, int, dict]] = []
     pending = list(range(K))
@@ -344,17 +353,19 @@ def transmission_kavg_adaptive(omega: float, device, lead_left, lead_right, kpoi
             break
         t, st = kb.run(float(eta), pending)
         nxt = []
-        for j, ki in enumerate(pending):
-            reason = _classify(t[j], st[j], max_allowed[ki], nonnegative_tolerance)
-            if reason is None:
-                accepted[ki] = (float(max(t[j], 0.0)), float(eta))
-            else:
-                kp = kpoints[ki]
-                attempts.append((ki, ei, {"omega": float(omega),
-                                          "kpar": tuple(float(x) for x in kp) if kp is not None else (),
-                                          "eta": float(eta), "t": None if reason == "exception" else float(t[j]),
-                                          "reason": reason}))
-                nxt.append(ki)
+        ok = _accepted(t, st, max_allowed, nonnegative_tolerance)
+        for ki, good, tj in zip(pending, ok.tolist(), t.tolist()):
+            if good:
+                accepted[ki] = (max(tj, 0.0), float(eta))
+        for j in np.nonzero(~ok)[0].tolist():
+            ki = pending[j]
+            reason = _classify(t[j], st[j], max_allowed, nonnegative_tolerance)
+            kp = kpoints[ki]
+            attempts.append((ki, ei, {"omega": float(omega),
+                                      "kpar": tuple(float(x) for x in kp) if kp is not None else (),
+                                      "eta": float(eta), "t": None if reason == "exception" else float(t[j]),
+                                      "reason": reason}))
+            nxt.append(ki)
         pending = nxt
     vals = [accepted[i][0] for i in range(K) if i in accepted]
     used = [accepted[i][1] for i in range(K) if i in accepted]
@@ -371,7 +382,7 @@ def transmission_kavg_adaptive(omega: float, device, lead_left, lead_right, kpoi
         "n_success": int(n_success),
         "n_failed": int(K - n_success),
         "success_fraction": success_fraction,
-        "eta_histogram": {float(e): int(sum(1 for u in used if u == float(e))) for e in eta_values},
+        "eta_histogram": {float(e): used.count(float(e)) for e in eta_values},
     }
     if collect_rejected:
         rej = [a[2] for a in sorted(attempts, key=lambda a: (a[0], a[1]))]
