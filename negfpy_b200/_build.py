@@ -42,13 +42,16 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     objdir = PKG / "_build"
     objdir.mkdir(exist_ok=True)
     flags = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-I", str(INCLUDE),
-                    "--expt-relaxed-constexpr", "-split-compile=0"]  # one optimiser thread per kernel instance
+                    "--expt-relaxed-constexpr"]
     objs = []
     procs = []
     for src in sources():
         obj = objdir / (src.stem + ".o")
         objs.append(obj)
-        cmd = [nvcc, *flags, "-c", str(src), "-o", str(obj)]
+        # One optimiser thread per kernel instance where a file holds many; the
+        # others keep their shared device functions in one unit.
+        split = ["-split-compile=0"] if src.stem.startswith("negf_mid") else []
+        cmd = [nvcc, *flags, *split, "-c", str(src), "-o", str(obj)]
         if verbose:
             print(" ".join(cmd), file=sys.stderr)
         procs.append((cmd, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT)))
