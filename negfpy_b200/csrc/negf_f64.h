@@ -118,6 +118,13 @@ int sgf_adj_launch(const SgfAdjArgs& sa, int np, int grid, double2* ws, cudaStre
 int full_grid(int np);
 size_t full_ws_bytes(int np, int n, int L, int grid);
 int full_launch(const FullArgs& fa, int np, int grid, double2* ws, cudaStream_t st);
+// Mixed and refined solve on mma.sync products, padded orders 16, 32, ..., 96.
+constexpr int kMaxOrder32 = 96;
+size_t mixed32_ws_bytes(int np, int n);
+size_t refine32_ws_bytes(int np, int n, int L);
+int mixed32_launch(const RgfArgs& a, int np, void* ws, size_t ws_bytes, cudaStream_t st);
+int refine32_launch(const RgfArgs& a, int np, void* ws, size_t ws_bytes, double tol, int maxit, int* steps_out,
+                    cudaStream_t st);
 }  // namespace mid
 // Block orders 49..256 (those above 104 padded to a multiple of 16): global-memory workspace.
 int global_order(int n);  // padded order for n > 48, 0 if unsupported

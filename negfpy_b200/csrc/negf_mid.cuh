@@ -62,13 +62,13 @@ __device__ __forceinline__ void load_left(AFrag& f, const Left& A, const Lane& L
   }
 }
 
-// c = op(A) op(X): A from global memory, X in shared memory.  The next chunk's
+// c = op(A) op(X), or c += with ADD: A from global memory, X in shared memory.  The next chunk's
 // A and the next column tile's B are loaded under the current tile's MMAs.
-template <class C, bool AC, bool BC>
+template <class C, bool AC, bool BC, bool ADD = false>
 __device__ __forceinline__ void prod(Acc<C>& c, const Left& A, const double2* X, int kch, const Lane& L) {
   int bb[2];
   smem::b_base<C, BC>(L, bb);
-  c.zero();
+  if (!ADD) c.zero();
   AFrag a, an, b, bn;
   load_left<AC>(a, A, L, 0);
   smem::load_b<C, BC>(b, X, bb, 0, 0);

@@ -137,12 +137,20 @@ int rgf_mixed_grid(int np) {
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   return nb * nsm;
 }
-size_t rgf_mixed_ws_bytes(int np, int n, int grid) { return (size_t)grid * mixed::mixed_ws_bytes_per_block(np, n); }
+// The same bytes on either product path, so that a workspace stays valid when the
+// path is set anew; the launch takes as many of its blocks as they hold.
+size_t rgf_mixed_ws_bytes(int np, int n, int grid) {
+  const size_t base = (size_t)grid * mixed::mixed_ws_bytes_per_block(np, n);
+  const size_t more = np <= mid::kMaxOrder32 ? mid::mixed32_ws_bytes(np, n) : 0;
+  return more > base ? more : base;
+}
 int rgf_mixed_launch(const RgfArgs& a, int np, int grid, void* ws, cudaStream_t st) {
   if (a.batch <= 0) return 0;
   if (mixed::use_tc(np)) {
     mixed::rgf_mixed_kernel<true><<<grid, mixed::kThreads, mixed::mixed_smem<true>(np), st>>>(
         a, np, static_cast<unsigned char*>(ws));
+  } else if (np <= mid::kMaxOrder32) {
+    return mid::mixed32_launch(a, np, ws, rgf_mixed_ws_bytes(np, a.n, grid), st);
   } else {
     mixed::rgf_mixed_kernel<false><<<grid, mixed::kThreads, mixed::mixed_smem<false>(np), st>>>(
         a, np, static_cast<unsigned char*>(ws));

@@ -381,7 +381,13 @@ int rgf_refine_grid(int np) {
   return nb * nsm;
 }
 size_t rgf_refine_ws_bytes(int np, int n, int L, int grid) {
-  return (size_t)grid * refine::ws_bytes_per_block(np, n, L);
+  // The same bytes on either product path, so that a workspace stays valid when
+  // the path is set anew.  The kernels of orders up to 96 use more blocks where
+  // their slots fit 2 GiB, and otherwise as many as these bytes hold.
+  const size_t base = (size_t)grid * refine::ws_bytes_per_block(np, n, L);
+  size_t more = np <= mid::kMaxOrder32 ? mid::refine32_ws_bytes(np, n, L) : 0;
+  if (more > ((size_t)2 << 30)) more = (size_t)2 << 30;
+  return more > base ? more : base;
 }
 int rgf_refine_launch(const RgfArgs& a, int np, int grid, void* ws, double tol, int maxit, int* steps_out,
                       cudaStream_t st) {
@@ -389,6 +395,8 @@ int rgf_refine_launch(const RgfArgs& a, int np, int grid, void* ws, double tol, 
   if (refine_use_tc(np)) {
     refine::rgf_refine_kernel<true><<<grid, refine::kThreads, refine::smem_bytes<true>(np), st>>>(
         a, np, static_cast<unsigned char*>(ws), tol, maxit, steps_out);
+  } else if (np <= mid::kMaxOrder32) {
+    return mid::refine32_launch(a, np, ws, rgf_refine_ws_bytes(np, a.n, a.L, grid), tol, maxit, steps_out, st);
   } else {
     refine::rgf_refine_kernel<false><<<grid, refine::kThreads, refine::smem_bytes<false>(np), st>>>(
         a, np, static_cast<unsigned char*>(ws), tol, maxit, steps_out);
