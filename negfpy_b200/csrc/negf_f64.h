@@ -126,6 +126,14 @@ int mixed32_launch(const RgfArgs& a, int np, void* ws, size_t ws_bytes, cudaStre
 int refine32_launch(const RgfArgs& a, int np, void* ws, size_t ws_bytes, double tol, int maxit, int* steps_out,
                     cudaStream_t st);
 }  // namespace mid
+// Decimation and device solve of orders 105..256: strips of a matrix in registers.
+namespace big {
+int grid(int np);
+size_t sr_ws_bytes(int np, int grid);
+size_t rgf_ws_bytes(int np, int n, int grid);
+int sr_launch(const SrArgs& a, int np, int grid, double2* ws, unsigned* counter, cudaStream_t st);
+int rgf_launch(const RgfArgs& a, int np, int grid, double2* ws, cudaStream_t st);
+}  // namespace big
 // Block orders 49..256 (those above 104 padded to a multiple of 16): global-memory workspace.
 int global_order(int n);  // padded order for n > 48, 0 if unsupported
 int sr_global_grid(int np);

@@ -1,28 +1,15 @@
-// FP64 kernels for block orders 105..256 (padded to NP, a multiple of 16), and
-// the adjoint and full-G kernels of these orders.
+// Adjoint and full-G kernels of block orders 105..256 (padded to NP, a multiple
+// of 16), and the dispatch by order of all FP64 kernels above order 48.
 //
-// Beyond n = 104 a block's registers do not hold a matrix, so here all of them
-// live in a per-block workspace in global memory (mostly L2 resident) and the
-// blocks are persistent: each takes points from an atomic counter.  The decimation and sweep kernels are register-capped for two
-// resident blocks per SM (128 registers a thread, a few hundred bytes of
-// spill), so one point's latency-bound pivot steps overlap another's
-// products: 1.22x (decimation) and 1.33x (sweep) faster at n = 96 than one
-// uncapped block per SM.
-// Row-major, row stride NP, no swizzle (global accesses of a warp fragment are
-// 16-byte loads from at most 8 rows).
-//
-//   sr_f64_global_kernel   Sancho-Rubio decimation, same recurrence, stopping
-//                          rule and outputs as sr_f64_kernel (negfpy
-//                          core/surface_gf.py:18-81).
-//   rgf_f64_global_kernel  Sigma, left-connected RGF sweep and trace, as
-//                          rgf_f64_kernel (negfpy core/negf.py:72-357).
-//
-// Products: each warp walks 16 x 16 output tiles (two m16n8 DMMA tiles) in
-// a strided loop; complex = four real mma.sync m16n8k8 f64.  Inversion:
-// blocked Gauss-Jordan, 8-column panels factored by the whole block in
-// shared memory with the division-free, look-ahead rule of the
-// shared-memory kernels, the rank-8 update of the whole matrix between two
-// global buffers on DMMA, and a final column gather.
+// All matrices live in a per-block workspace in global memory, row-major with
+// row stride NP; the blocks are persistent and take points from an atomic
+// counter.  Products: each warp walks 16 x 16 output tiles (two m16n8 DMMA
+// tiles) in a strided loop; complex = four real mma.sync m16n8k8 f64.
+// Inversion: blocked Gauss-Jordan, 8-column panels factored by the whole block in
+// shared memory with the division-free, look-ahead rule of the shared-memory
+// kernels, the rank-8 update of the whole matrix between two global buffers on
+// DMMA, and a final column gather.  The decimation and the device solve of these
+// orders are in negf_big.cu.
 #include <cstdio>
 
 #include "negf_common.cuh"
@@ -32,107 +19,6 @@
 
 namespace negf {
 namespace glob {
-
-// ------------------------------------------------------------ Sancho-Rubio --
-// Workspace per block: 7 NP x NP buffers (alpha, beta, eps, eps_s, three free).
-__global__ void __launch_bounds__(kThreads, 2) sr_f64_global_kernel(SrArgs a, int NP, double2* ws, unsigned* counter) {
-  extern __shared__ __align__(16) unsigned char smraw[];
-  const GJS sh = carve(smraw, NP);
-  double* red = reinterpret_cast<double*>(smraw + ((gjs_bytes(NP) + 15) / 16) * 16);
-  __shared__ int s_point;
-  const int n = a.n, tid = threadIdx.x;
-  const long long M2 = (long long)NP * NP;
-  double2* base = ws + (long long)blockIdx.x * 7 * M2;
-
-  for (;;) {
-    if (tid == 0) s_point = (int)atomicAdd(counter, 1u);
-    __syncthreads();
-    const int p = s_point;
-    __syncthreads();
-    if (p >= a.batch) break;
-    const long long kset = a.kidx ? (long long)a.kidx[p] : 0;
-    const double2* h00 = a.h00 + kset * a.lead_stride;
-    const double2* h01 = a.h01 + kset * a.lead_stride;
-    const double2* h10 = a.h10 ? a.h10 + kset * a.lead_stride : nullptr;
-    const double w = a.omega[p];
-    int it = 0;
-    double2* pg = nullptr;
-    const int status = sr_point(n, NP, h00, h01, h10, z_of(w, a.eta[p]), a.tol, a.maxiter, base, sh, red, &it, &pg);
-    if (status == kOk) {
-      if (a.g_out) {
-        double2* go = a.g_out + (long long)p * n * n;
-        for (int e = tid; e < n * n; e += kThreads) {
-          const int r = e / n, c = e - r * n;
-          go[e] = pg[(long long)r * NP + c];
-        }
-      }
-      if (a.dos_out) {
-        double t = 0.0;
-        for (int j = tid; j < n; j += kThreads) t += -2.0 * pg[(long long)j * NP + j].y;
-        t = block_sum(t, red);
-        if (tid == 0) a.dos_out[p] = (w / 3.141592653589793238462643383279502884) * t;
-      }
-    } else if (a.dos_out && tid == 0) {
-      a.dos_out[p] = __longlong_as_double(0x7ff8000000000000ULL);
-    }
-    if (tid == 0) {
-      if (a.iters_out) a.iters_out[p] = it;
-      if (a.status_out) a.status_out[p] = status;
-    }
-    __syncthreads();
-  }
-}
-
-// ---------------------------------------------------------------- RGF sweep --
-// Workspace per block: 6 NP x NP buffers (g, second inversion buffer, W, U,
-// G0, scratch) and Sigma_L, Sigma_R (n x n each).
-__global__ void __launch_bounds__(kThreads, 2) rgf_f64_global_kernel(RgfArgs a, int NP, double2* ws) {
-  extern __shared__ __align__(16) unsigned char smraw[];
-  const GJS sh = carve(smraw, NP);
-  double* red = reinterpret_cast<double*>(smraw + ((gjs_bytes(NP) + 15) / 16) * 16);
-  __shared__ int s_point;
-  const int n = a.n, tid = threadIdx.x;
-  const long long M2 = (long long)NP * NP;
-  double2* base = ws + (long long)blockIdx.x * (6 * M2 + 2LL * n * n);
-
-  for (;;) {
-    if (tid == 0) s_point = (int)atomicAdd(a.counter, 1u);
-    __syncthreads();
-    const int p = s_point;
-    __syncthreads();
-    if (p >= a.batch) break;
-    const int lst = a.lead_status ? a.lead_status[p] : 0;
-    if (lst != kOk) {
-      if (tid == 0) {
-        a.T_out[p] = __longlong_as_double(0x7ff8000000000000ULL);
-        if (a.status_out) a.status_out[p] = lst;
-      }
-      continue;
-    }
-    const long long k = a.kidx ? (long long)a.kidx[p] : 0;
-    RgfPoint q;
-    q.n = n;
-    q.nl = a.nl;
-    q.nr = a.nr;
-    q.L = a.L;
-    q.D = a.D + k * a.d_ks;
-    q.d_ls = a.d_ls;
-    q.C = a.C + k * a.c_ks;
-    q.c_ls = a.c_ls;
-    q.VL = a.VL + k * a.vl_ks;
-    q.VR = a.VR + k * a.vr_ks;
-    q.gL = a.gL + (long long)p * a.gl_ps;
-    q.gR = a.gR + (long long)p * a.gr_ps;
-    q.z = z_of(a.omega[p], a.eta_dev[p]);
-    double tval = 0.0;
-    const int status = rgf_point_f64(q, NP, base, sh, red, &tval);
-    if (tid == 0) {
-      a.T_out[p] = (status == kOk) ? tval : __longlong_as_double(0x7ff8000000000000ULL);
-      if (a.status_out) a.status_out[p] = status;
-    }
-    __syncthreads();
-  }
-}
 
 // ------------------------------------------------------- adjoint (gradient) --
 // Whole-matrix helpers over the (NP/16)^2 tiles of a block (each ends with a
@@ -705,24 +591,22 @@ static int occupancy_grid(K kernel, int np) {
 }  // namespace glob
 
 int sr_global_grid(int np) {
-  return np <= mid::kMaxOrder ? mid::sr_grid(np) : glob::occupancy_grid(glob::sr_f64_global_kernel, np);
+  return np <= mid::kMaxOrder ? mid::sr_grid(np) : big::grid(np);
 }
 int rgf_global_grid(int np) {
-  return np <= mid::kMaxOrder ? mid::rgf_grid(np) : glob::occupancy_grid(glob::rgf_f64_global_kernel, np);
+  return np <= mid::kMaxOrder ? mid::rgf_grid(np) : big::grid(np);
 }
 size_t sr_global_ws_bytes(int np, int grid) {
-  return np <= mid::kMaxOrder ? mid::sr_ws_bytes(np, grid) : (size_t)grid * 7 * np * np * 16;
+  return np <= mid::kMaxOrder ? mid::sr_ws_bytes(np, grid) : big::sr_ws_bytes(np, grid);
 }
 size_t rgf_global_ws_bytes(int np, int n, int grid) {
-  return np <= mid::kMaxOrder ? mid::rgf_ws_bytes(np, n, grid)
-                              : (size_t)grid * (6 * (size_t)np * np + 2 * (size_t)n * n) * 16;
+  return np <= mid::kMaxOrder ? mid::rgf_ws_bytes(np, n, grid) : big::rgf_ws_bytes(np, n, grid);
 }
 
 int sr_f64_global_launch(const SrArgs& a, int np, int grid, double2* ws, unsigned* counter, cudaStream_t st) {
   if (a.batch <= 0) return 0;
   if (np <= mid::kMaxOrder) return mid::sr_launch(a, np, grid, ws, counter, st);
-  glob::sr_f64_global_kernel<<<grid, glob::kThreads, glob::smem_bytes(np), st>>>(a, np, ws, counter);
-  return cudaGetLastError() == cudaSuccess ? 0 : -3;
+  return big::sr_launch(a, np, grid, ws, counter, st);
 }
 
 size_t grad_ws_bytes(int np, int n, int L, int grid) {
@@ -783,8 +667,7 @@ int grad_f64_launch(const GradArgs& ga, int np, int grid, double2* ws, cudaStrea
 int rgf_f64_global_launch(const RgfArgs& a, int np, int grid, double2* ws, cudaStream_t st) {
   if (a.batch <= 0) return 0;
   if (np <= mid::kMaxOrder) return mid::rgf_launch(a, np, grid, ws, st);
-  glob::rgf_f64_global_kernel<<<grid, glob::kThreads, glob::smem_bytes(np), st>>>(a, np, ws);
-  return cudaGetLastError() == cudaSuccess ? 0 : -3;
+  return big::rgf_launch(a, np, grid, ws, st);
 }
 
 }  // namespace negf

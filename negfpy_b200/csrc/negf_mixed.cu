@@ -1,7 +1,7 @@
 // Mixed-precision device solve: the RGF sweep in FP32 on the tensor cores,
 // the contact self-energies, broadenings and the trace in FP64.
 //
-// Same contract as rgf_f64_global_kernel (negfpy core/negf.py:72-357): per
+// Same contract as big::rgf_kernel (negfpy core/negf.py:72-357): per
 // point Sigma = V g V^H for both contacts from the FP64 surface GFs, the
 // left-connected sweep g_l = (z - D_l - C^H g_{l-1} C [- Sigma_R])^-1 with
 // G_{0,l} = G_{0,l-1} C g_l, and T = Re Tr[Gamma_L G Gamma_R G^H].

@@ -1,6 +1,5 @@
-// Per-point bodies of the global-workspace FP64 kernels, shared by the
-// single-system kernels (negf_f64_global.cu) and the uneven batch kernel
-// (negf_batch.cu).  Each function is executed by a whole thread block on one
+// Per-point bodies of the uneven batch kernel (negf_batch.cu) in FP64, parts of
+// which the mixed and refined device solves above order 96 share.  Each function is executed by a whole thread block on one
 // (omega, k) point, in workspace buffers the caller owns; every call ends
 // with the block synchronised.
 #pragma once

@@ -1,7 +1,7 @@
 // Refined device solve: the RGF factorisation in FP32 on the tensor cores,
 // corrected to FP64 accuracy by iterative refinement with FP64 residuals.
 //
-// Same contract as rgf_f64_global_kernel (negfpy core/negf.py:72-357): per
+// Same contract as big::rgf_kernel (negfpy core/negf.py:72-357): per
 // point Sigma = V g V^H of both contacts from the FP64 surface GFs, the
 // block-tridiagonal A = z - D - Sigma_L - Sigma_R, and
 // T = Re Tr[Gamma_L G_{0,L-1} Gamma_R G_{0,L-1}^H].  negfpy solves A X = E_R

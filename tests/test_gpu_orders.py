@@ -1,7 +1,7 @@
 """The one-point-per-block FP64 kernels at the edges of their tile splits.
 
 Orders just below, at and above each padded order (8, 16, 24, 32, 48, then
-every multiple of 8 up to 104, where the workspace kernels take over), leads
+every multiple of 8 up to 104, above it of 16), leads
 of another order than the device, layers with their own blocks, and both tile
 splits of order 9..16 (chosen by the number of points).  Random systems at an
 eta that keeps the decimation well conditioned, against the CPU oracle to the
@@ -70,6 +70,56 @@ def test_orders_match_oracle(n, nl, nr, layers):
         tr = O.transmission_point(w, s["on"], s["cp"], (*s["l"], None), (*s["r"], None), ETA, vl=s["vl"], vr=s["vr"],
                                   idx_l=np.arange(n), idx_r=np.arange(n * (layers - 1), n * layers))
         assert abs(t[i] - tr) <= TOL * max(abs(tr), 1.0)
+
+
+@pytest.mark.parametrize("n,nl,nr,layers,points", [
+    (106, 112, 60, 2, 3), (112, 112, 112, 1, 150), (113, 113, 113, 2, 150), (121, 128, 121, 3, 3), (128, 128, 128, 2, 150),
+    (129, 129, 129, 2, 3), (8, 150, 8, 2, 3), (161, 161, 100, 2, 3), (192, 192, 192, 2, 3), (193, 193, 193, 1, 3),
+    (225, 225, 225, 2, 3), (249, 256, 249, 2, 3), (256, 256, 256, 2, 3)])
+def test_large_orders_match_oracle(n, nl, nr, layers, points):
+    """Strips of 32 columns at their remainders, block sizes at the edges of their
+    classes, and up to order 128 both forms (chosen by the number of points)."""
+    s = _system(n, nl, nr, layers, seed=100 * n + nl)
+    omegas = np.resize([0.3, 1.1, 1.9], points)
+    g, dos, t, it = _solve(s, omegas)
+    for i, w in enumerate(omegas[:3]):
+        ref, nit = O.sancho_rubio(w, *s["l"], None, ETA)
+        assert it[i] == nit
+        assert np.max(np.abs(g[i] - ref)) <= TOL * np.max(np.abs(ref))
+        d = O.lead_surface_dos(w, *s["l"], None, ETA)
+        assert abs(dos[i] - d) <= 10 * TOL * max(abs(d), 1.0)
+        tr = O.transmission_point(w, s["on"], s["cp"], (*s["l"], None), (*s["r"], None), ETA, vl=s["vl"], vr=s["vr"],
+                                  idx_l=np.arange(n), idx_r=np.arange(n * (layers - 1), n * layers))
+        assert abs(t[i] - tr) <= TOL * max(abs(tr), 1.0)
+        for x in (g, dos, t, it):
+            assert all(np.array_equal(x[i], x[k]) for k in range(i, points, 3))
+
+
+@pytest.mark.parametrize("n,nl,nr,layers,points", [
+    (1, 2, 1, 2, 700), (15, 16, 9, 1, 700), (16, 16, 16, 3, 1300), (17, 20, 17, 2, 700), (32, 32, 32, 2, 800),
+    (33, 33, 30, 3, 500), (48, 48, 48, 2, 500), (49, 64, 49, 1, 40), (64, 64, 64, 3, 310), (65, 80, 65, 2, 40),
+    (80, 80, 80, 2, 40), (81, 96, 81, 3, 40), (96, 96, 96, 2, 160), (97, 97, 97, 2, 40)])
+def test_reduced_precision_orders(n, nl, nr, layers, points):
+    """The refined solve to the FP64 bound and the mixed one to its FP32-level
+    bound (1e-4) against the FP64 kernels, at the edges of the padded orders and
+    with more points than the launch holds blocks."""
+    s = _system(n, nl, nr, layers, seed=11 * n + nl)
+    c = lambda x: torch.as_tensor(x[None], device="cuda").contiguous()  # noqa: E731
+    om = torch.linspace(0.2, 2.2, points, dtype=torch.float64, device="cuda")
+    eta = torch.full_like(om, ETA)
+    ki = torch.zeros(points, dtype=torch.int32, device="cuda")
+    rl = engine.sgf_sr(c(s["l"][0]), c(s["l"][1]), None, om, eta, ki)
+    rr = engine.sgf_sr(c(s["r"][0]), c(s["r"][1]), None, om, eta, ki)
+    args = (c(np.stack(s["on"])), c(np.stack(s["cp"])) if layers > 1 else None, layers, c(s["vl"]), c(s["vr"]), rl["g"],
+            rr["g"], om, eta, ki, None)
+    t, st = engine.rgf_transmission(*args)
+    tm, sm = engine.rgf_transmission(*args, precision="mixed")
+    tr, sr, steps = engine.rgf_transmission_refine64(*args)
+    assert int(st.abs().sum()) == 0 and int(sm.abs().sum()) == 0 and int(sr.abs().sum()) == 0
+    scale = t.abs().clamp(min=1.0)
+    assert float(((tr - t).abs() / scale).max()) <= TOL
+    assert float(((tm - t).abs() / scale).max()) <= 1e-4
+    assert int(steps.min()) >= 1 and int(steps.max()) <= engine.REFINE_MAX_STEPS
 
 
 @pytest.mark.parametrize("n", [9, 12, 16])
