@@ -354,7 +354,9 @@ size_t negf_batch_workspace_bytes(int max_order, int precision, int blocks_per_s
   const int gmax = negf_batch_max_grid(max_order, precision, blocks_per_sm);
   if (gmax <= 0) return 0;
   const int g = (grid <= 0 || grid > gmax) ? gmax : grid;
-  return kCounterBytes + negf::batch_ws_bytes((max_order + 15) / 16 * 16, g);
+  const int npmax = (max_order + 15) / 16 * 16;
+  const size_t one = negf::batch_ws_bytes(npmax, g), two = negf::batch_split_ws_bytes(npmax, precision, blocks_per_sm, g);
+  return kCounterBytes + (two > one ? two : one);
 }
 
 int negf_batch_transmission(const NegfBatchSystem* systems, int n_systems, int max_order, const int* item_system,
@@ -379,11 +381,11 @@ int negf_batch_transmission(const NegfBatchSystem* systems, int n_systems, int m
     return fail(NEGF_EINVAL, "negf_batch_transmission: workspace missing or too small");
   if (n_items == 0) return 0;
   cudaStream_t st = as_stream(stream);
-  if (cudaMemsetAsync(workspace, 0, sizeof(unsigned int), st) != cudaSuccess)
+  if (cudaMemsetAsync(workspace, 0, 2 * sizeof(unsigned int), st) != cudaSuccess)
     return cuda_fail("negf_batch_transmission: counter reset");
   if (negf::batch_launch(systems, n_systems, item_system, item_k, item_omega, n_items, tol, maxiter, t_out,
                          status_out, iters_out, npmax, precision, blocks_per_sm, g, workspace,
-                         static_cast<char*>(workspace) + kCounterBytes, st) != 0)
+                         static_cast<char*>(workspace) + kCounterBytes, workspace_bytes - kCounterBytes, st) != 0)
     return cuda_fail("negf_batch_transmission");
   return 0;
 }

@@ -11,7 +11,7 @@ import torch
 
 pytestmark = pytest.mark.gpu
 
-from negfpy_b200 import engine, workloads as W  # noqa: E402
+from negfpy_b200 import _lib, engine, workloads as W  # noqa: E402
 from negfpy_b200.batch import Items, UnevenBatch  # noqa: E402
 
 TOL_T = 1e-10
@@ -169,3 +169,47 @@ def test_split_schedule_matches_single_launch(small, tmp_path):
     torch.cuda.synchronize()
     assert torch.equal(T3, single)
     b.release(g)
+
+
+@pytest.mark.parametrize("orders", [(24, 120, 192), (192,)])
+@pytest.mark.parametrize("blocks_per_sm", [1, 2])
+def test_batch_orders_above_128(orders, blocks_per_sm):
+    """Items above order 128 run in a kernel of their own beside the others; with
+    only the least workspace one kernel takes them all.  Out-of-range items of
+    both kinds, both against the per-system path; a captured launch replays."""
+    ws = W.uneven_workload(seed=3, n_systems=3, n_omega=4, k_range=(1, 3), layer_range=(2, 5), orders=orders)
+    b = UnevenBatch(ws)
+    it = b.items([w.omegas for w in ws], "lpt")
+    ref = _reference(ws)
+    r = b.solve(it, "f64", blocks_per_sm=blocks_per_sm)
+    assert int((r["status"] != 0).sum()) == 0
+    assert float(((r["T"] - ref).abs() / ref.abs().clamp_min(1.0)).max()) <= TOL_T
+    lib, mo = _lib.load(), b.max_order
+    grid = b.max_grid("f64", blocks_per_sm)
+    if mo > 128:  # the least workspace: 11 padded matrices a block, and the counters
+        T, st, iters = b._buffers(it.system.numel())
+        least = 256 + grid * 11 * ((mo + 15) // 16 * 16) ** 2 * 16
+        space = torch.empty(least, dtype=torch.uint8, device="cuda")
+        _lib.check(lib.negf_batch_transmission(
+            b.table.data_ptr(), b.n_systems, mo, it.system.data_ptr(), it.k.data_ptr(), it.omega.data_ptr(),
+            it.system.numel(), 1e-12, 200, 0, blocks_per_sm, 0, T.data_ptr(), st.data_ptr(), iters.data_ptr(),
+            space.data_ptr(), least, _lib.stream_handle(None)), "negf_batch_transmission")
+        for got, key in ((T, "T"), (st, "status"), (iters, "iters")):
+            out = torch.empty_like(got)
+            out[it.perm] = got
+            assert torch.equal(out, r[key])
+    big = int(np.argmax([w.lead_l["d00"].shape[-1] for w in ws]))
+    bad = Items(torch.cat([it.system, torch.tensor([99, big, big], dtype=torch.int32, device="cuda")]),
+                torch.cat([it.k, torch.tensor([0, 1000, -1], dtype=torch.int32, device="cuda")]),
+                torch.cat([it.omega, it.omega[:3]]), torch.arange(it.system.numel() + 3, device="cuda"),
+                np.concatenate([it.cost, np.zeros(3)]))
+    T, st, _ = b.launch(bad, "f64", blocks_per_sm=blocks_per_sm)
+    assert st[-3:].tolist() == [_lib.BAD_ITEM] * 3 and bool(torch.isnan(T[-3:]).all())
+    assert int((st[:-3] != 0).sum()) == 0
+    g, (Tg, sg, ig) = b.graph(it, "f64", blocks_per_sm=blocks_per_sm)
+    Tg.zero_()
+    g.replay()
+    torch.cuda.synchronize()
+    out = torch.empty_like(Tg)
+    out[it.perm] = Tg
+    assert torch.equal(out, r["T"])
