@@ -388,14 +388,19 @@ typedef struct NegfBatchSystem {
  * for that many resident blocks (0 on a bad argument). */
 int negf_batch_max_grid(int max_order, int precision, int blocks_per_sm);
 
-/* Workspace bytes of negf_batch_transmission (grid <= 0: the largest grid). */
+/*
+ * Workspace bytes of negf_batch_transmission (grid <= 0: the largest grid).  In
+ * FP64 with max_order above 128 this is what the kernel for the items above 128
+ * and the one for the rest need together; with less, down to 11 padded complex
+ * matrices of max_order a block, one kernel takes every item.
+ */
 size_t negf_batch_workspace_bytes(int max_order, int precision, int blocks_per_sm, int grid);
 
 /* sizeof(NegfBatchSystem), for bindings that lay the table out themselves. */
 size_t negf_batch_system_bytes(void);
 
 /*
- * Uneven batch in one persistent launch: item i is system item_system[i] of
+ * Uneven batch in one call of persistent kernels: item i is system item_system[i] of
  * the device-memory table `systems` at its k set item_k[i] and frequency
  * item_omega[i].  Per item: the lead decimation(s) of negf_sgf_sr_f64 and the
  * device solve of negf_rgf_transmission_f64 (precision 0) or of
