@@ -14,6 +14,9 @@
 // fragments (10 bytes per clock and SM).  An inverse factors 32 columns at a
 // time in registers and applies their four updates to each other strip in one
 // pass over it, so that the matrix crosses L2 n / 32 times.
+// Decimation / 6-layer sweep at n = 192, ms, before and after: 148 points 109 / 24.8
+// -> 51.8 / 10.8, 296 points 125 / 27.5 -> 98.6 / 21.6 (products at 0.77 of the FP64
+// pipe, the inverse's strips at 0.45, its pivot steps latency).
 // Every element keeps its sequence of operations (chunks of 8, panels of 8), so
 // results are bitwise those of the kernels of the smaller orders.
 #pragma once
