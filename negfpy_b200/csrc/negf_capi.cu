@@ -1,5 +1,6 @@
 // extern "C" entry points of libnegfb200.so (declared in include/negf_b200.h).
 // Argument checks happen here, on the host; the kernels assume valid input.
+#include <cstdint>
 #include <cstdio>
 #include <cstring>
 
@@ -20,6 +21,11 @@ int cuda_fail(const char* where) {
 }
 inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 constexpr size_t kCounterBytes = 256;
+// The matrices behind the counters, at a 32-byte boundary whatever the workspace's
+// own alignment (the kernels of orders above 104 access pairs of elements).
+inline double2* matrices(void* workspace) {
+  return reinterpret_cast<double2*>((reinterpret_cast<uintptr_t>(workspace) + kCounterBytes) & ~(uintptr_t)31);
+}
 }  // namespace
 
 namespace negf {
@@ -79,8 +85,7 @@ int negf_sgf_sr_f64(int n, int batch, const double* h00, const double* h01, cons
     if (cudaMemsetAsync(workspace, 0, sizeof(unsigned int), st) != cudaSuccess)
       return cuda_fail("negf_sgf_sr_f64: counter reset");
     const int grc = negf::sr_f64_global_launch(a, np, grid,
-                                               reinterpret_cast<double2*>(static_cast<char*>(workspace) + kCounterBytes),
-                                               reinterpret_cast<unsigned*>(workspace), st);
+                                               matrices(workspace), reinterpret_cast<unsigned*>(workspace), st);
     if (grc != 0) return cuda_fail("negf_sgf_sr_f64 (global)");
     return 0;
   }
@@ -167,7 +172,7 @@ int negf_rgf_transmission_f64(int n_dev, int n_lead_l, int n_lead_r, int n_layer
   a.T_out = t_out;
   a.status_out = status_out;
   a.counter = reinterpret_cast<unsigned int*>(workspace);
-  a.sigma_ws = reinterpret_cast<double2*>(static_cast<char*>(workspace) + kCounterBytes);
+  a.sigma_ws = matrices(workspace);
   cudaStream_t st = as_stream(stream);
   if (np != 1 && cudaMemsetAsync(workspace, 0, sizeof(unsigned int), st) != cudaSuccess)
     return cuda_fail("negf_rgf_transmission_f64: counter reset");
@@ -385,7 +390,7 @@ int negf_batch_transmission(const NegfBatchSystem* systems, int n_systems, int m
     return cuda_fail("negf_batch_transmission: counter reset");
   if (negf::batch_launch(systems, n_systems, item_system, item_k, item_omega, n_items, tol, maxiter, t_out,
                          status_out, iters_out, npmax, precision, blocks_per_sm, g, workspace,
-                         static_cast<char*>(workspace) + kCounterBytes, workspace_bytes - kCounterBytes, st) != 0)
+                         matrices(workspace), workspace_bytes - kCounterBytes, st) != 0)
     return cuda_fail("negf_batch_transmission");
   return 0;
 }

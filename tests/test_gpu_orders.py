@@ -12,7 +12,7 @@ import numpy as np
 import pytest
 import torch
 
-from negfpy_b200 import engine
+from negfpy_b200 import _lib, engine
 from oracle import negf_oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -93,6 +93,35 @@ def test_large_orders_match_oracle(n, nl, nr, layers, points):
         assert abs(t[i] - tr) <= TOL * max(abs(tr), 1.0)
         for x in (g, dos, t, it):
             assert all(np.array_equal(x[i], x[k]) for k in range(i, points, 3))
+
+
+@pytest.mark.parametrize("n", [96, 120, 150])
+@pytest.mark.parametrize("shift", [16, 240])
+def test_workspace_at_any_16_byte_boundary(n, shift):
+    """A workspace that starts 16 bytes off a 32-byte boundary gives the same
+    surface GF and T as an aligned one."""
+    s = _system(n, n, n, 2, seed=n)
+    c = lambda x: torch.as_tensor(x[None], device="cuda").contiguous()  # noqa: E731
+    om = torch.tensor([0.3, 1.1, 1.9], dtype=torch.float64, device="cuda")
+    eta = torch.full_like(om, ETA)
+    ki = torch.zeros(3, dtype=torch.int32, device="cuda")
+    h00, h01, on, cp = c(s["l"][0]), c(s["l"][1]), c(np.stack(s["on"])), c(np.stack(s["cp"]))
+    vl, vr = c(s["vl"]), c(s["vr"])
+    ref = engine.sgf_sr(h00, h01, None, om, eta, ki)
+    tref, _ = engine.rgf_transmission(on, cp, 2, vl, vr, ref["g"], ref["g"], om, eta, ki, None)
+    lib, ptr = _lib.load(), _lib.ptr
+    need = [int(lib.negf_sgf_workspace_bytes(n)), int(lib.negf_rgf_workspace_bytes(n, n, n))]
+    ws = torch.empty(max(need) + 512, dtype=torch.uint8, device="cuda")
+    off = -ws.data_ptr() % 256 + shift
+    g, t = torch.empty_like(ref["g"]), torch.empty_like(tref)
+    st, it = torch.empty_like(ki), torch.empty_like(ki)
+    _lib.check(lib.negf_sgf_sr_f64(n, 3, ptr(h00), ptr(h01), None, 0, ptr(ki), ptr(om), ptr(eta), 1e-12, 200, ptr(g), None,
+                                   ptr(it), ptr(st), ptr(ws[off:]), need[0], _lib.stream_handle(None)), "negf_sgf_sr_f64")
+    _lib.check(lib.negf_rgf_transmission_f64(
+        n, n, n, 2, 3, ptr(on), 0, n * n, ptr(cp), 0, n * n, ptr(vl), 0, ptr(vr), 0, ptr(g), n * n, ptr(g), n * n, ptr(ki),
+        ptr(om), ptr(eta), None, ptr(t), ptr(st), ptr(ws[off:]), need[1], _lib.stream_handle(None)),
+        "negf_rgf_transmission_f64")
+    assert torch.equal(g, ref["g"]) and torch.equal(t, tref)
 
 
 @pytest.mark.parametrize("n,nl,nr,layers,points", [
