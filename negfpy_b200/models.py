@@ -14,6 +14,7 @@ reused for every frequency, instead of once per (omega, k) point.
 
 from __future__ import annotations
 
+import operator
 from dataclasses import dataclass
 
 import numpy as np
@@ -146,8 +147,9 @@ def material_kspace_stack(params: MaterialKspaceParams, kpoints: list, layer_mas
     Returns ``{"d00","d01","d10"}: [K, n, n]`` for the lead, and when
     ``n_layers`` is given also ``"onsite": [K, L, n, n]`` and
     ``"coupling": [K, L-1, n, n]`` for the device (per-layer masses from
-    ``layer_masses`` of shape ``(L, n_atoms)``).  The arithmetic is the same
-    as the per-k builders of negfpy ``models/material_kspace.py:99-193``.
+    ``layer_masses`` of shape ``(L, n_atoms)``: the first ``n_layers`` rows, an
+    ``IndexError`` if there are fewer).  The arithmetic is the same as the
+    per-k builders of negfpy ``models/material_kspace.py:99-193``.
     """
     kk = [parse_ky_kz(k) for k in kpoints]
     ky = np.array([a for a, _ in kk], dtype=float)
@@ -167,11 +169,16 @@ def material_kspace_stack(params: MaterialKspaceParams, kpoints: list, layer_mas
         "d10": m[None, :, None] * phi10 * m[None, None, :],
     }
     if n_layers is not None:
+        n_layers = operator.index(n_layers)
         if layer_masses is None:
             lm = np.repeat(np.asarray(params.masses, dtype=float)[None, :], n_layers, axis=0)
         else:
             lm = np.asarray(layer_masses, dtype=float)
-        ms = 1.0 / np.sqrt(np.repeat(lm, params.dof_per_atom, axis=1))  # [L, n]
+        if n_layers <= 0:
+            raise ValueError("n_layers must be positive.")
+        if lm.shape[0] < n_layers:
+            raise IndexError(f"layer_masses has {lm.shape[0]} rows for n_layers = {n_layers}.")
+        ms = 1.0 / np.sqrt(np.repeat(lm[:n_layers].reshape(n_layers, -1), params.dof_per_atom, axis=1))  # [L, n]
         out["onsite"] = ms[None, :, :, None] * phi00[:, None] * ms[None, :, None, :]
         out["coupling"] = ms[None, :-1, :, None] * phi01[:, None] * ms[None, 1:, None, :]
     return out
