@@ -144,13 +144,16 @@ __device__ __forceinline__ void store_rows(double2* G, const Acc<C>& c, const La
 #pragma unroll
     for (int q = 0; q < 2; ++q) G[L.r0 * C::NP + L.c0 + 8 * j + q] = c.get(0, j, q);
 }
-// The warp's rows of X -> row-major workspace.
+// The warp's rows of X -> row-major workspace.  Ends with the warp synchronised: a
+// lane writes other elements than those it owns, and the next step may read the
+// rows as a left operand or element by element.
 template <class C>
 __device__ __forceinline__ void copy_rows(double2* G, const double2* X, const Lane& L) {
   for (int e = threadIdx.x & 31; e < 8 * C::NP; e += 32) {
     const int r = L.R0 + e / C::NP, c = e % C::NP;
     G[r * C::NP + c] = X[sidx<C::NP>(r, c)];
   }
+  __syncwarp();
 }
 
 // ------------------------------------------------------------ Sancho-Rubio --
@@ -475,7 +478,6 @@ __global__ void __launch_bounds__(C::NTH, C::OCC) rgf_kernel(RgfArgs a, double2*
         prod<C, false, false>(c, u, X, kch, L);
         store_rows<C>(G0, c, L);
       }
-      __syncwarp();
     }
     __syncthreads();
     double tval = 0.0;

@@ -235,3 +235,28 @@ def test_adjoint_and_full_green_orders(n, nl, nr, layers):
     h00 = gl @ lam @ gl
     assert near(ad["h00"][0].cpu(), h00)
     assert near(ad["h01"][0].cpu(), gl @ h01.mH @ h00 + (h00 @ h01 @ gl).mH)
+
+
+@pytest.mark.parametrize("n", [3, 16, 23, 32, 48, 64, 72, 80, 96, 104])
+@pytest.mark.parametrize("layers", [1, 2])
+def test_last_diagonal_block_of_full_green(n, layers):
+    """G_{L-1,L-1} is read back by other lanes than wrote it: many points, every
+    padded order, equal points bitwise equal and the block the oracle's to 1e-10."""
+    s = _system(n, n, n, layers, seed=31 * n + layers)
+    distinct, points = 3, 600
+    c = lambda x: torch.as_tensor(x[None], device="cuda").contiguous()  # noqa: E731
+    om = torch.tensor(np.resize([0.3, 1.1, 1.9], points), device="cuda")
+    eta = torch.full_like(om, ETA)
+    ki = torch.zeros(points, dtype=torch.int32, device="cuda")
+    rl = engine.sgf_sr(c(s["l"][0]), c(s["l"][1]), None, om, eta, ki)
+    rr = engine.sgf_sr(c(s["r"][0]), c(s["r"][1]), None, om, eta, ki)
+    g, sl, sr, st = engine.device_green(c(np.stack(s["on"])), c(np.stack(s["cp"])) if layers > 1 else None, layers,
+                                        c(s["vl"]), c(s["vr"]), rl["g"], rr["g"], om, eta, ki, None)
+    assert int(st.abs().sum()) == 0
+    sl, sr = sl.cpu(), sr.cpu()
+    on = {"on": [torch.as_tensor(b) for b in s["on"]], "cp": [torch.as_tensor(b) for b in s["cp"]]}
+    for i in range(distinct):
+        same = g[i::distinct]
+        assert torch.equal(same, same[:1].expand_as(same))
+        ref = torch.linalg.inv(_dense(on, (float(om[i]) + 1j * ETA) ** 2, sl[i], sr[i]))[-n:, -n:]
+        assert float((g[i, -n:, -n:].cpu() - ref).abs().max()) <= TOL * float(ref.abs().max())
