@@ -390,9 +390,9 @@ int negf_batch_max_grid(int max_order, int precision, int blocks_per_sm);
 
 /*
  * Workspace bytes of negf_batch_transmission (grid <= 0: the largest grid).  In
- * FP64 with max_order above 128 this is what the kernel for the items above 128
- * and the one for the rest need together; with less, down to 11 padded complex
- * matrices of max_order a block, one kernel takes every item.
+ * FP64 with max_order above 128 (blocks_per_sm 2: 144) this is what the kernel for
+ * the items above it and the one for the rest need together; with less, down to 11
+ * padded complex matrices of max_order a block, one kernel takes every item.
  */
 size_t negf_batch_workspace_bytes(int max_order, int precision, int blocks_per_sm, int grid);
 

@@ -13,7 +13,7 @@
 // up to 256; the per-block workspace and the shared memory are sized for the
 // largest order in the batch.
 //
-// In FP64 with orders above 128 in the batch, those items run first in a kernel
+// In FP64 with orders above kSplit in the batch, those items run first in a kernel
 // of their own on the strips of negf_big.cuh (one block per SM, which two blocks
 // of the other kernel cannot join), and the kernel for the rest is launched as
 // its programmatic dependent: its blocks take the SMs as the first kernel's run
@@ -47,10 +47,16 @@ struct BatchArgs {
   int* status_out;
   int* iters_out;
   unsigned* counter;
-  int big_order;   // items of order kSplit + 1 .. big_order belong to the other kernel (0: none)
+  int split, big_order;  // items of order split + 1 .. big_order run in big_kernel (big_order 0: none)
   bool dependent;  // launched as the other kernel's programmatic dependent
 };
-constexpr int kSplit = 128;
+// The largest order that stays with the smaller items.  One block an SM: the strips
+// are faster from 129 on (135 and 144: 0.91-0.97 of the time).  Two: at 129..144
+// the second block hides more than the strips save (ms, strips / two blocks: 296
+// items of order 144 67.2 / 64.8, 520 of 135 122.6 / 115.6), above not (296 items
+// of 150 74.7 / 81.4, of 192 115.5 / 145.5).
+template <int MINB>
+constexpr int kSplit = MINB == 2 ? 144 : 128;
 
 __host__ __device__ inline int pad16(int n) { return (n + 15) / 16 * 16; }
 // Per-block workspace, in complex128 elements, for padded order NP: the two
@@ -99,7 +105,7 @@ __global__ void __launch_bounds__(kThreads, MINB) batch_kernel(BatchArgs a, int 
     const double w = a.item_omega[p];
     const int n = d.n_dev, nl = d.n_lead_l, nr = d.n_lead_r;
     const int top = max(n, max(nl, nr));
-    if (top > kSplit && top <= a.big_order) continue;
+    if (top > a.split && top <= a.big_order) continue;
     int status = bad_item(d, k, NPmax) ? kBadItem : kOk, iters = 0;
     // 1. lead surface GFs (compact, row stride = lead order)
     for (int side = 0; side < 2 && status == kOk; ++side) {
@@ -163,7 +169,7 @@ __global__ void __launch_bounds__(kThreads, MINB) batch_kernel(BatchArgs a, int 
   if (a.dependent && blockIdx.x == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
-// The items of order kSplit + 1 .. a.big_order.  Workspace per block: the lead
+// The items of order a.split + 1 .. a.big_order.  Workspace per block: the lead
 // surface GFs and the scratch of the decimation (7 NP^2; the device solve needs
 // less).
 __host__ __device__ inline size_t big_elems(int np) { return 9 * (size_t)np * np; }
@@ -185,7 +191,7 @@ __global__ void __launch_bounds__(NT, 1) big_kernel(BatchArgs a, int NPmax, doub
     if (si < 0 || si >= a.n_systems) continue;
     const NegfBatchSystem& d = a.sys[si];
     const int top = max(d.n_dev, max(d.n_lead_l, d.n_lead_r));
-    if (top <= kSplit || top > a.big_order) continue;
+    if (top <= a.split || top > a.big_order) continue;
     const long long k = a.item_k[p];
     const double w = a.item_omega[p];
     int status = bad_item(d, k, a.big_order) ? kBadItem : kOk, iters = 0;
@@ -293,7 +299,7 @@ int launch_big(const BatchArgs& a, int npmax, int grid, double2* ws, cudaStream_
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 
-// Blocks of the two kernels of an FP64 batch with orders above kSplit.
+// Blocks of the two kernels of an FP64 batch with orders above kSplit<MINB>.
 struct Split {
   int big, rest;
 };
@@ -302,23 +308,27 @@ Split split_grids(int grid) {
   int dev = 0, nsm = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  const int gmax = max_grid<false, MINB>(kSplit);
+  const int gmax = max_grid<false, MINB>(kSplit<MINB>);
   return {grid < nsm ? grid : nsm, grid < gmax ? grid : gmax};
 }
-size_t split_elems(const Split& g, int npmax) { return g.big * big_elems(npmax) + g.rest * block_elems(kSplit); }
+template <int MINB>
+size_t split_elems(const Split& g, int npmax) {
+  return g.big * big_elems(npmax) + g.rest * block_elems(kSplit<MINB>);
+}
 // Their launches; 1 when the workspace is too small for both (one kernel then
 // takes every item).  The counters are neighbours, both zero.
 template <int MINB>
 int launch_split(BatchArgs a, int npmax, int grid, double2* ws, size_t ws_bytes, cudaStream_t st) {
   const Split g = split_grids<MINB>(grid);
   if (g.big <= 0 || g.rest <= 0) return -3;
-  if (split_elems(g, npmax) * 16 > ws_bytes) return 1;
+  if (split_elems<MINB>(g, npmax) * 16 > ws_bytes) return 1;
+  a.split = kSplit<MINB>;
   a.big_order = npmax;
   const int rc = npmax <= 192 ? launch_big<384>(a, npmax, g.big, ws, st) : launch_big<512>(a, npmax, g.big, ws, st);
   if (rc != 0) return rc;
   a.counter += 1;
   a.dependent = true;
-  return launch_variant<false, MINB>(a, kSplit, g.rest, ws + g.big * big_elems(npmax), st);
+  return launch_variant<false, MINB>(a, kSplit<MINB>, g.rest, ws + g.big * big_elems(npmax), st);
 }
 
 }  // namespace batch
@@ -329,8 +339,9 @@ int batch_max_grid(int npmax, int mixed, int minb) {
 }
 size_t batch_ws_bytes(int npmax, int grid) { return (size_t)grid * batch::block_elems(npmax) * 16; }
 size_t batch_split_ws_bytes(int npmax, int mixed, int minb, int grid) {
-  if (mixed || npmax <= batch::kSplit) return 0;
-  return 16 * batch::split_elems(minb == 2 ? batch::split_grids<2>(grid) : batch::split_grids<1>(grid), npmax);
+  if (mixed || npmax <= (minb == 2 ? batch::kSplit<2> : batch::kSplit<1>)) return 0;
+  return 16 * (minb == 2 ? batch::split_elems<2>(batch::split_grids<2>(grid), npmax)
+                         : batch::split_elems<1>(batch::split_grids<1>(grid), npmax));
 }
 int batch_launch(const NegfBatchSystem* sys, int n_systems, const int* item_system, const int* item_k, const double* item_omega,
                  int n_items, double tol, int maxiter, double* t_out, int* status_out, int* iters_out, int npmax,
@@ -348,10 +359,10 @@ int batch_launch(const NegfBatchSystem* sys, int n_systems, const int* item_syst
   a.status_out = status_out;
   a.iters_out = iters_out;
   a.counter = static_cast<unsigned*>(counter);
-  a.big_order = 0;
+  a.split = a.big_order = 0;
   a.dependent = false;
   double2* w = static_cast<double2*>(ws);
-  if (!mixed && npmax > batch::kSplit) {
+  if (!mixed && npmax > (minb == 2 ? batch::kSplit<2> : batch::kSplit<1>)) {
     const int rc = minb == 2 ? batch::launch_split<2>(a, npmax, grid, w, ws_bytes, st)
                              : batch::launch_split<1>(a, npmax, grid, w, ws_bytes, st);
     if (rc <= 0) return rc;

@@ -168,7 +168,7 @@ int tc_cgemm_launch(int np, int batch, const float2* a, const float2* b, float2*
 // Uneven batch (negf_batch.cu).
 int batch_max_grid(int npmax, int mixed, int minb);
 size_t batch_ws_bytes(int npmax, int grid);                              // the least it needs
-size_t batch_split_ws_bytes(int npmax, int mixed, int minb, int grid);  // for both kernels of orders above 128
+size_t batch_split_ws_bytes(int npmax, int mixed, int minb, int grid);  // for both kernels of a split batch
 int batch_launch(const ::NegfBatchSystem* sys, int n_systems, const int* item_system, const int* item_k,
                  const double* item_omega, int n_items, double tol, int maxiter, double* t_out, int* status_out,
                  int* iters_out, int npmax, int mixed, int minb, int grid, void* counter, void* ws, size_t ws_bytes,

@@ -213,3 +213,30 @@ def test_batch_orders_above_128(orders, blocks_per_sm):
     out = torch.empty_like(Tg)
     out[it.perm] = Tg
     assert torch.equal(out, r["T"])
+
+
+@pytest.mark.parametrize("shapes", [((6, 8),), ((5, 10),), ((2, 4), (5, 9), (6, 8), (5, 10))])  # 144; 150; 24, 135, 144, 150
+@pytest.mark.parametrize("blocks_per_sm", [1, 2])
+def test_batch_split_line(shapes, blocks_per_sm):
+    """Which items leave the common kernel: above order 128 with one block an SM,
+    above 144 with two (up to it the call needs no more workspace than that
+    kernel's 11 padded matrices a block).  Both against the per-system path."""
+    ws = []
+    for i, (ny, nz) in enumerate(shapes):
+        p, kps = W.spring_network(40 + i, ny, nz), W.kgrid(2)
+        st = W.material_kspace_stack(p, kps, n_layers=1)
+        lead = {x: st[x] for x in ("d00", "d01", "d10")}
+        wmax = W.estimate_omega_max(p, nk=2)
+        ws.append(W.Workload(f"s{i}", np.array([0.31, 0.57]) * wmax, kps, lead, lead, st["onsite"], st["d01"][:, None], 3,
+                             eta=1e-6 * wmax * wmax, uniform_layers=True))
+    b = UnevenBatch(ws)
+    r = b.solve(b.items([w.omegas for w in ws]), "f64", blocks_per_sm=blocks_per_sm)
+    ref = _reference(ws)
+    assert int((r["status"] != 0).sum()) == 0
+    assert float(((r["T"] - ref).abs() / ref.abs().clamp_min(1.0)).max()) <= TOL_T
+    one = 256 + b.max_grid("f64", blocks_per_sm) * 11 * ((b.max_order + 15) // 16 * 16) ** 2 * 16
+    need = b.workspace_bytes("f64", blocks_per_sm)
+    if blocks_per_sm == 2 and b.max_order <= 144:
+        assert need == one
+    else:
+        assert need >= one
