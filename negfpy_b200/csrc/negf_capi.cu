@@ -400,7 +400,7 @@ size_t negf_device_green_workspace_bytes(int n_dev, int n_lead_l, int n_lead_r, 
   const int nmax = max3(n_dev, n_lead_l, n_lead_r);
   if (nmax > 256) return 0;
   const int np = negf::adj_order(nmax);
-  const int grid = negf::full_grid(np);
+  const int grid = negf::full_grid(np, n_dev, n_layers);
   if (grid <= 0) return 0;
   return kCounterBytes + negf::full_ws_bytes(np, n_dev, n_layers, grid);
 }
@@ -425,7 +425,7 @@ int negf_device_green_f64(int n_dev, int n_lead_l, int n_lead_r, int n_layers, i
   const int nmax = max3(n_dev, n_lead_l, n_lead_r);
   if (nmax > 256) return fail(NEGF_EUNSUPPORTED, "negf_device_green_f64: block order above 256");
   const int np = negf::adj_order(nmax);
-  const int grid = negf::full_grid(np);
+  const int grid = negf::full_grid(np, n_dev, n_layers);
   if (grid <= 0) return cuda_fail("negf_device_green_f64: occupancy query");
   if (!workspace || workspace_bytes < kCounterBytes + negf::full_ws_bytes(np, n_dev, n_layers, grid))
     return fail(NEGF_EINVAL, "negf_device_green_f64: workspace missing or too small");
@@ -476,7 +476,7 @@ size_t negf_adjoint_workspace_bytes(int n_dev, int n_lead_l, int n_lead_r, int n
   const int nmax = max3(n_dev, n_lead_l, n_lead_r);
   if (nmax > 256) return 0;
   const int np = negf::adj_order(nmax);
-  const int grid = negf::grad_grid(np);
+  const int grid = negf::grad_grid(np, n_dev, n_layers);
   if (grid <= 0) return 0;
   return kCounterBytes + negf::grad_ws_bytes(np, n_dev, n_layers, grid);
 }
@@ -517,7 +517,7 @@ static int rgf_adjoint_common(const char* name, int n_dev, int n_lead_l, int n_l
   const int nmax = max3(n_dev, n_lead_l, n_lead_r);
   if (nmax > 256) return fail2(NEGF_EUNSUPPORTED, name, "block order above 256");
   const int np = negf::adj_order(nmax);
-  const int grid = negf::grad_grid(np);
+  const int grid = negf::grad_grid(np, n_dev, n_layers);
   if (grid <= 0) return cuda_fail2(name, "occupancy query");
   if (!workspace || workspace_bytes < kCounterBytes + negf::grad_ws_bytes(np, n_dev, n_layers, grid))
     return fail2(NEGF_EINVAL, name, "workspace missing or too small");

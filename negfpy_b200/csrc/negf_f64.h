@@ -109,13 +109,13 @@ size_t sr_ws_bytes(int np, int grid);
 size_t rgf_ws_bytes(int np, int n, int grid);
 int sr_launch(const SrArgs& a, int np, int grid, double2* ws, unsigned* counter, cudaStream_t st);
 int rgf_launch(const RgfArgs& a, int np, int grid, double2* ws, cudaStream_t st);
-int grad_grid(int np);
+int grad_grid(int np, int n, int L);
 size_t grad_ws_bytes(int np, int n, int L, int grid);
 int grad_launch(const GradArgs& ga, int np, int grid, double2* ws, cudaStream_t st);
 int sgf_adj_grid(int np);
 size_t sgf_adj_ws_bytes(int np, int grid);
 int sgf_adj_launch(const SgfAdjArgs& sa, int np, int grid, double2* ws, cudaStream_t st);
-int full_grid(int np);
+int full_grid(int np, int n, int L);
 size_t full_ws_bytes(int np, int n, int L, int grid);
 int full_launch(const FullArgs& fa, int np, int grid, double2* ws, cudaStream_t st);
 // Mixed and refined solve on mma.sync products, padded orders 16, 32, ..., 96.
@@ -177,11 +177,11 @@ int batch_launch(const ::NegfBatchSystem* sys, int n_systems, const int* item_sy
 // Adjoints and full G: np = adj_order(largest order), 0 if unsupported.
 int adj_order(int n);
 size_t full_ws_bytes(int np, int n, int L, int grid);
-int full_grid(int np);
+int full_grid(int np, int n, int L);
 int full_f64_launch(const FullArgs& fa, int np, int grid, double2* ws, cudaStream_t st);
 
 size_t grad_ws_bytes(int np, int n, int L, int grid);
-int grad_grid(int np);
+int grad_grid(int np, int n, int L);
 int grad_f64_launch(const GradArgs& ga, int np, int grid, double2* ws, cudaStream_t st);
 
 size_t sgf_adj_ws_bytes(int np, int grid);

@@ -613,8 +613,8 @@ size_t grad_ws_bytes(int np, int n, int L, int grid) {
   if (np <= mid::kMaxOrder) return mid::grad_ws_bytes(np, n, L, grid);
   return (size_t)grid * ((14 + 2 * (size_t)L) * np * np + 2 * (size_t)n * n) * 16;
 }
-int grad_grid(int np) {
-  if (np <= mid::kMaxOrder) return mid::grad_grid(np);
+int grad_grid(int np, int n, int L) {
+  if (np <= mid::kMaxOrder) return mid::grad_grid(np, n, L);
   const int g = glob::occupancy_grid(glob::rgf_grad_f64_kernel, np);
   int dev = 0, nsm = 0;
   cudaGetDevice(&dev);
@@ -625,8 +625,8 @@ size_t full_ws_bytes(int np, int n, int L, int grid) {
   if (np <= mid::kMaxOrder) return mid::full_ws_bytes(np, n, L, grid);
   return (size_t)grid * ((6 + 3 * (size_t)L) * np * np + 2 * (size_t)n * n) * 16;
 }
-int full_grid(int np) {
-  if (np <= mid::kMaxOrder) return mid::full_grid(np);
+int full_grid(int np, int n, int L) {
+  if (np <= mid::kMaxOrder) return mid::full_grid(np, n, L);
   const int g = glob::occupancy_grid(glob::rgf_full_f64_kernel, np);
   int dev = 0, nsm = 0;
   cudaGetDevice(&dev);

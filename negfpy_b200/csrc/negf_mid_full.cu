@@ -7,8 +7,8 @@
 namespace negf {
 namespace mid {
 
-int full_grid(int np) {
-  return with_adj(np, [](auto c) { return grid_of<decltype(c)>(); });
+int full_grid(int np, int n, int L) {
+  return with_adj(np, [&](auto c) { return slots_of<decltype(c)>(full_ws<decltype(c)>(n, L)); });
 }
 size_t full_ws_bytes(int np, int n, int L, int grid) {
   return with_adj(np, [&](auto c) { return (size_t)grid * full_ws<decltype(c)>(n, L) * 16; });

@@ -5,8 +5,8 @@
 namespace negf {
 namespace mid {
 
-int grad_grid(int np) {
-  return with_adj(np, [](auto c) { return grid_of<decltype(c)>(); });
+int grad_grid(int np, int n, int L) {
+  return with_adj(np, [&](auto c) { return slots_of<decltype(c)>(grad_ws<decltype(c)>(n, L)); });
 }
 size_t grad_ws_bytes(int np, int n, int L, int grid) {
   return with_adj(np, [&](auto c) { return (size_t)grid * grad_ws<decltype(c)>(n, L) * 16; });

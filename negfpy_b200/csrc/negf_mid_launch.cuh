@@ -21,6 +21,17 @@ static int grid_of() {
   }
   return n * C::OCC;
 }
+// Blocks of a kernel that keeps matrices of every layer: all that are resident at
+// once while their workspace fits 512 MiB, else no more than two an SM, which
+// bounds what a long device takes (full G, n = 32, 40 layers: 0.6 GB instead of
+// 1.2).  Two cost the adjoint of 2368 points 1.17 times the time of four at n = 32
+// and 1.46 at 16 (6 layers: 3.14 -> 3.68 ms, 0.76 -> 1.12), that of 296 nothing.
+template <class C>
+static int slots_of(size_t elems_per_block) {
+  const int g = grid_of<C>();
+  if (C::OCC <= 2 || g <= 0 || (size_t)g * elems_per_block * 16 <= ((size_t)512 << 20)) return g;
+  return g / C::OCC * 2;
+}
 // The kernel's dynamic shared memory limit, raised once per device.
 template <auto kernel, class C>
 static int raise_smem() {
