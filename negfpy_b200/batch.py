@@ -139,18 +139,13 @@ class UnevenBatch:
 
     @staticmethod
     def _record(s: engine.StackedSystem, eta: float, eta_dev: float) -> NegfBatchSystem:
-        K, Lo, n, _ = s.onsite.shape
+        K, _, n, _ = s.onsite.shape
+        (on_ks, on_ls), cp, (cp_ks, cp_ls) = engine.layer_strides(s.onsite, s.coupling, s.n_layers)
         r = NegfBatchSystem()
         r.n_dev, r.n_lead_l, r.n_lead_r, r.n_layers, r.n_k = n, s.nl, s.nr, s.n_layers, K
         r.same_leads = 1 if s.same_leads else 0
-        r.onsite, r.onsite_kstride, r.onsite_lstride = s.onsite.data_ptr(), (Lo * n * n if K > 1 else 0), (
-            0 if Lo == 1 else n * n)
-        if s.coupling is None or s.n_layers == 1:
-            r.coupling, r.coupling_kstride, r.coupling_lstride = None, 0, 0
-        else:
-            Kc, Lc = s.coupling.shape[0], s.coupling.shape[1]
-            r.coupling = s.coupling.data_ptr()
-            r.coupling_kstride, r.coupling_lstride = (Lc * n * n if Kc > 1 else 0), (0 if Lc == 1 else n * n)
+        r.onsite, r.onsite_kstride, r.onsite_lstride = s.onsite.data_ptr(), on_ks, on_ls
+        r.coupling, r.coupling_kstride, r.coupling_lstride = None if cp is None else cp.data_ptr(), cp_ks, cp_ls
         r.v_left, r.v_left_kstride = s.vl.data_ptr(), (n * s.nl if s.vl.shape[0] > 1 else 0)
         r.v_right, r.v_right_kstride = s.vr.data_ptr(), (n * s.nr if s.vr.shape[0] > 1 else 0)
         for side, lead in (("l", s.lead_l), ("r", s.lead_r)):

@@ -84,6 +84,25 @@ def sgf_sr(d00: torch.Tensor, d01: torch.Tensor, d10: torch.Tensor | None, omega
     return {"g": g, "dos": dos, "iters": iters, "status": status}
 
 
+def layer_strides(onsite: torch.Tensor, coupling: torch.Tensor | None, n_layers: int):
+    """(k, layer) strides of the onsite blocks, the coupling (None where there is
+    none to read) and its strides, in complex elements.  One block serves every
+    layer; fewer than the layers need, but more than one, is a ``ValueError``
+    (the kernels would read past them)."""
+    n = int(onsite.shape[-1])
+
+    def strides(t, need, name):
+        count = int(t.shape[1])
+        if count != 1 and count < need:
+            raise ValueError(f"{name} holds blocks of {count} layers; n_layers = {n_layers} needs 1 or {need}")
+        return count * n * n if t.shape[0] > 1 else 0, 0 if count == 1 else n * n
+
+    on = strides(onsite, int(n_layers), "onsite")
+    if coupling is None or n_layers == 1:
+        return on, None, (0, 0)
+    return on, coupling, strides(coupling, int(n_layers) - 1, "coupling")
+
+
 _ws_cache: dict = {}
 
 
@@ -112,20 +131,14 @@ def rgf_transmission(onsite: torch.Tensor, coupling: torch.Tensor | None, n_laye
         raise ValueError(f"unknown precision {precision!r}; expected 'f64' or 'mixed'")
     lib = _lib.load()
     dev = _dev()
-    K, Lo, n, _ = onsite.shape
+    n = int(onsite.shape[-1])
     nl, nr = int(vl.shape[-1]), int(vr.shape[-1])
     P = int(omega.shape[0])
     T = torch.empty(P, dtype=RDT, device=dev)
     st = torch.empty(P, dtype=torch.int32, device=dev)
     if P == 0:
         return T, st
-    on_ks = Lo * n * n if K > 1 else 0
-    on_ls = 0 if Lo == 1 else n * n
-    if coupling is None or n_layers == 1:
-        cp, cp_ks, cp_ls = None, 0, 0
-    else:
-        Kc, Lc = coupling.shape[0], coupling.shape[1]
-        cp, cp_ks, cp_ls = coupling, (Lc * n * n if Kc > 1 else 0), (0 if Lc == 1 else n * n)
+    (on_ks, on_ls), cp, (cp_ks, cp_ls) = layer_strides(onsite, coupling, n_layers)
     vl_ks = n * nl if vl.shape[0] > 1 else 0
     vr_ks = n * nr if vr.shape[0] > 1 else 0
     mixed = precision == "mixed"
@@ -157,7 +170,7 @@ def rgf_transmission_refine64(onsite, coupling, n_layers, vl, vr, gl, gr, omega,
     ``_lib.REFINE_FAIL`` (no fallback here)."""
     lib = _lib.load()
     dev = _dev()
-    K, Lo, n, _ = onsite.shape
+    n = int(onsite.shape[-1])
     nl, nr = int(vl.shape[-1]), int(vr.shape[-1])
     P = int(omega.shape[0])
     T = torch.empty(P, dtype=RDT, device=dev)
@@ -165,13 +178,7 @@ def rgf_transmission_refine64(onsite, coupling, n_layers, vl, vr, gl, gr, omega,
     steps = torch.zeros(P, dtype=torch.int32, device=dev)
     if P == 0:
         return T, st, steps
-    on_ks = Lo * n * n if K > 1 else 0
-    on_ls = 0 if Lo == 1 else n * n
-    if coupling is None or n_layers == 1:
-        cp, cp_ks, cp_ls = None, 0, 0
-    else:
-        Kc, Lc = coupling.shape[0], coupling.shape[1]
-        cp, cp_ks, cp_ls = coupling, (Lc * n * n if Kc > 1 else 0), (0 if Lc == 1 else n * n)
+    (on_ks, on_ls), cp, (cp_ks, cp_ls) = layer_strides(onsite, coupling, n_layers)
     need = int(lib.negf_rgf_refined_workspace_bytes(n, nl, nr, int(n_layers)))
     if need == 0:
         raise RuntimeError(f"block order {max(n, nl, nr)} is not supported by the refined kernel")
@@ -248,7 +255,7 @@ def device_green(onsite: torch.Tensor, coupling: torch.Tensor | None, n_layers: 
     (``negf_device_green_f64``); blocks as in ``rgf_transmission``."""
     lib = _lib.load()
     dev = _dev()
-    K, Lo, n, _ = onsite.shape
+    n = int(onsite.shape[-1])
     nl, nr = int(vl.shape[-1]), int(vr.shape[-1])
     P = int(omega.shape[0])
     dim = int(n_layers) * n
@@ -258,13 +265,7 @@ def device_green(onsite: torch.Tensor, coupling: torch.Tensor | None, n_layers: 
     st = torch.empty(P, dtype=torch.int32, device=dev)
     if P == 0:
         return G, sl, sr, st
-    on_ks = Lo * n * n if K > 1 else 0
-    on_ls = 0 if Lo == 1 else n * n
-    if coupling is None or n_layers == 1:
-        cp, cp_ks, cp_ls = None, 0, 0
-    else:
-        Kc, Lc = coupling.shape[0], coupling.shape[1]
-        cp, cp_ks, cp_ls = coupling, (Lc * n * n if Kc > 1 else 0), (0 if Lc == 1 else n * n)
+    (on_ks, on_ls), cp, (cp_ks, cp_ls) = layer_strides(onsite, coupling, n_layers)
     need = int(lib.negf_device_green_workspace_bytes(n, nl, nr, int(n_layers)))
     if need == 0:
         raise RuntimeError(f"block order {max(n, nl, nr)} is not supported by the device Green's function kernel")
@@ -536,6 +537,7 @@ class StackedSystem:
             vr = lr[1]
             if vr.shape[-2] != n:
                 raise ValueError("default right coupling needs the device block order to equal the lead's")
+        layer_strides(on, cp, n_layers)
         return cls(ll, lr, on, cp, int(n_layers), _c(vl, dev), _c(vr, dev), bool(same_leads))
 
     def transmission(self, omega: torch.Tensor, k_index: torch.Tensor, eta: torch.Tensor,
