@@ -42,9 +42,12 @@ def _r(t, device=None) -> torch.Tensor:
 def _upload(arrays, device) -> list:
     """``_c`` of several host arrays (None stays None): small ones go to the
     device in one copy and come back as views of it (each copy from pageable
-    memory costs about 10 us of host time)."""
+    memory costs about 10 us of host time).  What ``_c`` refuses is refused at any
+    size."""
     host = [a if isinstance(a, torch.Tensor) or a is None else np.asarray(a) for a in arrays]
     small = [i for i, a in enumerate(host) if isinstance(a, np.ndarray) and a.size <= 1 << 14]
+    for i in small:
+        torch.as_tensor(host[i])  # raises for the types and strides torch has no tensor of
     out = [None if a is None else a if i in small else _c(a, device) for i, a in enumerate(host)]
     if small:
         flat = torch.from_numpy(np.concatenate([host[i].astype(np.complex128, copy=False).ravel() for i in small]))

@@ -42,3 +42,14 @@ def test_a_shared_lead_gives_the_same_system():
     assert negf._same_lead(a["lead_l"], a["lead_r"]) and negf._same_lead(b["lead_l"], b["lead_r"])
     for key in ("vl", "vr", "onsite", "coupling"):
         assert np.array_equal(a[key], b[key])
+
+
+@pytest.mark.parametrize("bad", ["object", ">f8", "longdouble", "clongdouble", "datetime64[s]", "U8", "reversed"])
+@pytest.mark.parametrize("size", [3, 200])
+def test_upload_refuses_what_a_conversion_refuses(bad, size):
+    a = np.arange(float(size * size)).reshape(size, size)
+    a = a[::-1] if bad == "reversed" else a.astype(bad)
+    with pytest.raises((TypeError, ValueError)) as ref:
+        engine._c(a, torch.device("cpu"))
+    with pytest.raises(ref.type):
+        engine._upload([np.ones((2, 2)), a], torch.device("cpu"))
