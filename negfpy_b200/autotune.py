@@ -8,8 +8,8 @@ blocks finish: "lpt" (largest estimated cost first), "interleave"
 (round-robin over systems) or "system" (system by system).  The tuner times
 every (blocks_per_sm, order) pair on a small omega sample of the batch with
 CUDA events, keeps the fastest, and caches the choice in a JSON file keyed by
-the GPU, the precision and the shape of the batch (block orders, layer counts
-and k counts of its systems).
+the GPU, the kernels' sources, the precision and the shape of the batch (block
+orders, layer counts and k counts of its systems).
 
 ``BatchTuner.tune_split`` makes the same choice per padded-order class for
 the split schedule (one launch per class), so the launch shape and item
@@ -27,6 +27,7 @@ Cache file: ``$NEGF_B200_TUNE_CACHE``, else ``~/.cache/negfpy_b200/autotune.json
 
 from __future__ import annotations
 
+import functools
 import hashlib
 import json
 import os
@@ -34,6 +35,8 @@ from pathlib import Path
 from typing import Callable
 
 import numpy as np
+
+from . import _build
 
 CANDIDATES = [(bps, order) for bps in (1, 2) for order in ("lpt", "interleave", "system")]
 
@@ -43,9 +46,21 @@ def default_cache_path() -> Path:
     return Path(env) if env else Path.home() / ".cache" / "negfpy_b200" / "autotune.json"
 
 
+@functools.cache
+def kernel_revision() -> str:
+    """Digest of the CUDA sources (of the built library where they are not
+    shipped): a choice timed with other kernels does not count for these."""
+    files = sorted(p for p in _build.CSRC.glob("*") if p.suffix in (".cu", ".cuh", ".h")) or [_build.LIB]
+    h = hashlib.sha1()
+    for p in files:
+        h.update(p.name.encode() + b"\0" + p.read_bytes())
+    return h.hexdigest()
+
+
 def batch_signature(shapes, precision: str, gpu: str) -> str:
-    """Stable key of a batch: GPU name, precision and the sorted (n, nl, nr, L, K, same_leads) shapes."""
-    body = json.dumps({"gpu": gpu, "precision": precision, "shapes": sorted(list(map(list, shapes)))})
+    """Stable key of a batch: GPU name, kernels, precision and the sorted (n, nl, nr, L, K, same_leads) shapes."""
+    body = json.dumps({"gpu": gpu, "kernels": kernel_revision(), "precision": precision,
+                       "shapes": sorted(list(map(list, shapes)))})
     return hashlib.sha1(body.encode()).hexdigest()
 
 

@@ -122,3 +122,23 @@ def test_sum_by_k_groups_points_in_order():
     none = torch.zeros((1, 2, 3), dtype=torch.complex128)
     _sum_by_k(none, src, None)
     assert torch.equal(none, one)
+
+
+def test_a_choice_timed_with_other_kernels_is_timed_again(tmp_path, monkeypatch):
+    from negfpy_b200 import _build, autotune
+
+    shapes = [(48, 48, 48, 20, 64, 1)]
+    tuner = BatchTuner(tmp_path / "tune.json")
+    first = tuner.select(batch_signature(shapes, "f64", "gpu"), lambda b, o: float(b))
+    assert not first["cached"] and tuner.select(batch_signature(shapes, "f64", "gpu"), lambda b, o: 1.0)["cached"]
+    (tmp_path / "csrc").mkdir()
+    (tmp_path / "csrc" / "a.cu").write_text("// other kernels\n")
+    monkeypatch.setattr(_build, "CSRC", tmp_path / "csrc")
+    autotune.kernel_revision.cache_clear()
+    try:
+        again = tuner.select(batch_signature(shapes, "f64", "gpu"), lambda b, o: -float(b))
+        assert not again["cached"] and again["blocks_per_sm"] == 2
+    finally:
+        monkeypatch.undo()
+        autotune.kernel_revision.cache_clear()
+    assert tuner.select(batch_signature(shapes, "f64", "gpu"), lambda b, o: 1.0)["blocks_per_sm"] == 1
