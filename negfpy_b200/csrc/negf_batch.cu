@@ -47,7 +47,7 @@ struct BatchArgs {
   int* status_out;
   int* iters_out;
   unsigned* counter;
-  int split, big_order;  // items of order split + 1 .. big_order run in big_kernel (big_order 0: none)
+  int big_order;   // items of order kSplit + 1 .. big_order run in big_kernel (0: none)
   bool dependent;  // launched as the other kernel's programmatic dependent
 };
 // The largest order that stays with the smaller items.  One block an SM: the strips
@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(kThreads, MINB) batch_kernel(BatchArgs a, int 
     const double w = a.item_omega[p];
     const int n = d.n_dev, nl = d.n_lead_l, nr = d.n_lead_r;
     const int top = max(n, max(nl, nr));
-    if (top > a.split && top <= a.big_order) continue;
+    if (top > kSplit<MINB> && top <= a.big_order) continue;
     int status = bad_item(d, k, NPmax) ? kBadItem : kOk, iters = 0;
     // 1. lead surface GFs (compact, row stride = lead order)
     for (int side = 0; side < 2 && status == kOk; ++side) {
@@ -169,11 +169,11 @@ __global__ void __launch_bounds__(kThreads, MINB) batch_kernel(BatchArgs a, int 
   if (a.dependent && blockIdx.x == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
-// The items of order a.split + 1 .. a.big_order.  Workspace per block: the lead
+// The items of order SPLIT + 1 .. a.big_order.  Workspace per block: the lead
 // surface GFs and the scratch of the decimation (7 NP^2; the device solve needs
 // less).
 __host__ __device__ inline size_t big_elems(int np) { return 9 * (size_t)np * np; }
-template <int NT>
+template <int NT, int SPLIT>
 __global__ void __launch_bounds__(NT, 1) big_kernel(BatchArgs a, int NPmax, double2* ws) {
   extern __shared__ __align__(16) unsigned char smraw[];
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(NT, 1) big_kernel(BatchArgs a, int NPmax, doub
     if (si < 0 || si >= a.n_systems) continue;
     const NegfBatchSystem& d = a.sys[si];
     const int top = max(d.n_dev, max(d.n_lead_l, d.n_lead_r));
-    if (top <= a.split || top > a.big_order) continue;
+    if (top <= SPLIT || top > a.big_order) continue;
     const long long k = a.item_k[p];
     const double w = a.item_omega[p];
     int status = bad_item(d, k, a.big_order) ? kBadItem : kOk, iters = 0;
@@ -284,18 +284,18 @@ int launch_variant(const BatchArgs& a, int npmax, int grid, double2* ws, cudaStr
   return cudaLaunchKernelEx(&cfg, batch_kernel<MIXED, MINB>, a, npmax, ws) == cudaSuccess ? 0 : -3;
 }
 
-template <int NT>
+template <int NT, int SPLIT>
 int launch_big(const BatchArgs& a, int npmax, int grid, double2* ws, cudaStream_t st) {
   static std::atomic<bool> done[64];
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -3;
   if (!done[dev].load(std::memory_order_acquire)) {
-    if (cudaFuncSetAttribute(big_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if (cudaFuncSetAttribute(big_kernel<NT, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)big::shared_bytes<2>(NT / 2)) != cudaSuccess)
       return -3;
     done[dev].store(true, std::memory_order_release);
   }
-  big_kernel<NT><<<grid, 2 * npmax, big::shared_bytes<2>(npmax), st>>>(a, npmax, ws);
+  big_kernel<NT, SPLIT><<<grid, 2 * npmax, big::shared_bytes<2>(npmax), st>>>(a, npmax, ws);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 
@@ -322,9 +322,9 @@ int launch_split(BatchArgs a, int npmax, int grid, double2* ws, size_t ws_bytes,
   const Split g = split_grids<MINB>(grid);
   if (g.big <= 0 || g.rest <= 0) return -3;
   if (split_elems<MINB>(g, npmax) * 16 > ws_bytes) return 1;
-  a.split = kSplit<MINB>;
   a.big_order = npmax;
-  const int rc = npmax <= 192 ? launch_big<384>(a, npmax, g.big, ws, st) : launch_big<512>(a, npmax, g.big, ws, st);
+  const int rc = npmax <= 192 ? launch_big<384, kSplit<MINB>>(a, npmax, g.big, ws, st)
+                              : launch_big<512, kSplit<MINB>>(a, npmax, g.big, ws, st);
   if (rc != 0) return rc;
   a.counter += 1;
   a.dependent = true;
@@ -359,7 +359,7 @@ int batch_launch(const NegfBatchSystem* sys, int n_systems, const int* item_syst
   a.status_out = status_out;
   a.iters_out = iters_out;
   a.counter = static_cast<unsigned*>(counter);
-  a.split = a.big_order = 0;
+  a.big_order = 0;
   a.dependent = false;
   double2* w = static_cast<double2*>(ws);
   if (!mixed && npmax > (minb == 2 ? batch::kSplit<2> : batch::kSplit<1>)) {
