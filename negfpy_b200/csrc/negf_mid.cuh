@@ -401,15 +401,11 @@ __device__ __forceinline__ double trace_t(const double2* sigL, const double2* si
 
 // Workspace: g, G_{0,l}, U (row-major), Sigma_L, Sigma_R.
 template <class C>
-struct Park {
-  static constexpr int kNeed = Eps<C>::kWarps * C::PARK * 8;
-  static constexpr int kCols = kNeed <= 32 ? 32 : kNeed <= 64 ? 64 : kNeed <= 128 ? 128 : kNeed <= 256 ? 256 : 512;
-};
-template <class C>
 constexpr size_t rgf_ws(int n) { return 3 * (size_t)C::MAT + 2 * (size_t)n * n; }
 
 template <class C>
 __global__ void __launch_bounds__(C::NTH, C::OCC) rgf_kernel(RgfArgs a, double2* ws) {
+  static_assert(C::PARK == 0, "no Tensor Memory here");
   constexpr int NP = C::NP, MAT = C::MAT;
   extern __shared__ __align__(16) unsigned char smraw[];
   double2* const X = reinterpret_cast<double2*>(smraw);
@@ -418,13 +414,6 @@ __global__ void __launch_bounds__(C::NTH, C::OCC) rgf_kernel(RgfArgs a, double2*
   const Lane L = smem::lane_geo<C>();
   double2* const Gl = ws + (long long)blockIdx.x * rgf_ws<C>(n);
   double2 *const G0 = Gl + MAT, *const U = G0 + MAT, *const sigL = U + MAT, *const sigR = sigL + (long long)n * n;
-  uint32_t park = 0;
-  if (C::PARK) {
-    if (tid < 32) umma::tmem_alloc(&sh.tmem, Park<C>::kCols);
-    __syncthreads();
-    umma::fence_after_sync();
-    park = sh.tmem + ((uint32_t)(tid >> 5 & 3) << 21) + (uint32_t)(tid >> 7) * (C::PARK * 8);
-  }
   const Left gl{Gl, NP, NP, NP}, g0{G0, NP, NP, NP}, u{U, NP, NP, NP};
 
   for (;;) {
@@ -468,7 +457,7 @@ __global__ void __launch_bounds__(C::NTH, C::OCC) rgf_kernel(RgfArgs a, double2*
       if (l == 0) load_tiles<C>(c, sigL, n, L);
       minus_d<C>(c, D + (long long)l * a.d_ls, l == nlay - 1 ? sigR : nullptr, z, n, L);
       __syncthreads();  // every read of W is done
-      status = smem::gj_invert<C>(c, X, X, n, L, sh.gj, park);
+      status = smem::gj_invert<C>(c, X, X, n, L, sh.gj);
       if (status != kOk) break;
       // g_l, and G_{0,0} = g_0, G_{0,l} = U g_l
       if (l + 1 < nlay) copy_rows<C>(Gl, X, L);
@@ -491,7 +480,6 @@ __global__ void __launch_bounds__(C::NTH, C::OCC) rgf_kernel(RgfArgs a, double2*
     }
     __syncthreads();
   }
-  if (C::PARK && tid < 32) umma::tmem_dealloc(sh.tmem, Park<C>::kCols);
 }
 
 }  // namespace mid
