@@ -1,5 +1,7 @@
 """Uneven batches: many independent systems of different block orders, layer
-counts and k grids solved in ONE persistent launch (``negf_batch_transmission``).
+counts and k grids solved in one call of persistent kernels
+(``negf_batch_transmission``: one kernel, or in FP64 with orders above 128, with two
+blocks an SM above 144, one for those and one for the rest).
 
 Each system is a lead/device/lead problem of negfpy's path (``core/negf.py:306-357``
 per (omega, k)); an item is (system, k index, omega).  The host
@@ -8,7 +10,7 @@ per (omega, k)); an item is (system, k index, omega).  The host
   table of ``NegfBatchSystem`` records the kernel reads,
 * orders the items (by default largest estimated cost first, so that the
   persistent blocks finish together),
-* launches once, optionally inside a CUDA graph that is replayed for repeated
+* makes that call, optionally inside a CUDA graph that is replayed for repeated
   solves of the same items,
 * for ``precision="mixed_fallback"`` re-solves in FP64 the items whose FP32
   device sweep failed.  (The batch kernel has no iterative refinement: its
@@ -212,7 +214,7 @@ class UnevenBatch:
 
     def launch(self, it: Items, precision: str = "f64", grid: int = 0, tol: float = 1e-12, maxiter: int = 200,
                out=None, stream=None, blocks_per_sm: int = 1, max_order: int = 0, ws=None):
-        """One persistent launch over the items (launch order).  Returns
+        """One call over the items (launch order).  Returns
         (T, status, iters) in launch order.  ``max_order``: the largest block
         order among the items' systems (default: the batch's); ``ws``: a
         workspace of at least ``workspace_bytes`` (default: the cached one)."""
@@ -235,7 +237,7 @@ class UnevenBatch:
 
     def graph(self, it: Items, precision: str = "f64", grid: int = 0, tol: float = 1e-12, maxiter: int = 200,
               blocks_per_sm: int = 1):
-        """A CUDA graph of the launch over ``it`` (counter reset + one kernel) and
+        """A CUDA graph of the launch over ``it`` (counter reset and its kernels) and
         its output buffers; ``g.replay()`` re-solves the items."""
         P = int(it.system.numel())
         out = self._buffers(P)

@@ -9,9 +9,9 @@
 // streamed the whole matrix through L2 in each of the n / 8 updates of an
 // inverse (64 bytes per clock and SM): about half the FP64 pipe.  Here warp w
 // owns rows 16 w .. 16 w + 15.  A product keeps a 32-column strip of its result
-// in registers, stages the strip of its right operand through a ring in shared
-// memory once per block and reads each row of the left operand straight into
-// fragments (10 bytes per clock and SM).  An inverse factors 32 columns at a
+// in registers and takes both operands through a ring in shared memory, filled by
+// cp.async four chunks ahead (at full FP64 rate 8 bytes per clock and SM of the left
+// one, 256 / n of the right one).  An inverse factors 32 columns at a
 // time in registers and applies their four updates to each other strip in one
 // pass over it, so that the matrix crosses L2 n / 32 times.
 // Decimation / 6-layer sweep at n = 192, ms, before and after: 148 points 109 / 24.8

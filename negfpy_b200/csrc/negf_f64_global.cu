@@ -673,6 +673,7 @@ int rgf_f64_global_launch(const RgfArgs& a, int np, int grid, double2* ws, cudaS
 }  // namespace negf
 
 namespace negf {
+// The padded orders with_adj() has splits for, then multiples of 16.
 int adj_order(int n) {
   if (n <= 0 || n > 256) return 0;
   for (int np : {16, 24, 32, 48, 64, 72, 80, 96, 104})

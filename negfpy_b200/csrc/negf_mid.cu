@@ -5,10 +5,16 @@
 // fastest of those measured.  1024 points, L = 20, decimation / device solve in
 // ms: n = 54 9.2 / 7.2, n = 63 12.0 / 9.6, n = 72 21.3 / 16.3, n = 75 26.1 /
 // 20.9, n = 84 32.5 / 25.5, n = 96 38.7 / 30.5.  Two blocks share an SM up to
-// order 72 (83 KB of shared memory and 72 accumulator registers each); above, a
-// second block does not fit.  Parking tiles takes the pivot steps of the
-// decimation from 745 to 600 cycles at n = 96 (spills); the device solve does
-// not gain from it.
+// order 72 (83 KB of shared memory each); above, a second block does not fit.
+// Parking tiles takes the pivot steps of the decimation from 745 to 600 cycles at
+// n = 96 (spills); the device solve does not gain from it.
+//
+// Registers a thread follow from the warps a scheduler holds: 168 for three, 128
+// for four, 96 for five, so orders 72 (two blocks of nine warps put five on one
+// scheduler) and 104 (thirteen warps, four) spill where their neighbours hardly
+// do.  Bytes stored / loaded a thread, decimation and device solve: 72 1676 / 1288
+// and 1820 / 1860, 104 1428 / 1120 and 2144 / 2188; the other orders at most 40 / 56
+// and 212 / 360.
 #include "negf_mid_launch.cuh"
 
 namespace negf {

@@ -12,6 +12,8 @@ namespace mid {
 // block's phases leave units idle that another's use (n = 48, 888 points, 20
 // layers: three blocks 11.6 ms, two 12.8; n = 63, 1776 points, 8 layers: two 17.9,
 // one 22.4).  Orders 80 and 96: shared memory allows one or two, registers one.
+// The refined solve still spills 1452 / 1460 bytes a thread (stored / loaded) at 48
+// and 1240 / 1260 at 96, the mixed one 568 / 644 and 676 / 684.
 template <class F>
 static auto with32(int np, F&& f) {
   switch (np) {

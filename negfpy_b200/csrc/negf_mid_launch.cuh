@@ -45,7 +45,16 @@ static int raise_smem() {
   return 0;
 }
 
-// f with the split of an adj_order() up to kMaxOrder.
+// f with the split of an adj_order() up to kMaxOrder: the padded orders of the
+// decimation without 40, 56 and 88.  Those three are not built; orders 33..40,
+// 49..56 and 81..88 run on the next split, and the missing ones would take 0.82,
+// 0.86 and 0.90 of its time (adjoint, full G and surface-GF adjoint at 40, 56, 88
+// against 48, 64, 96; 148 to 1184 points).
+//
+// Blocks per SM as for the decimation, four up to order 32.  Spills as there:
+// the adjoint of the device solve stores / loads 5056 / 6580 bytes a thread at 72 and
+// 5476 / 6160 at 104, 512 / 960 or less elsewhere; the full G 2044 / 2116 and
+// 2324 / 2512, the surface-GF adjoint 1288 / 1616 and 1864 / 2108.
 template <class F>
 static auto with_adj(int np, F&& f) {
   switch (np) {

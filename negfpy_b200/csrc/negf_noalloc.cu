@@ -102,8 +102,9 @@ int negf_rgf_transmission_f64_noalloc(int n_dev, int n_lead_l, int n_lead_r, int
     if (grid <= 0) return noalloc_fail(NEGF_ECUDA, "negf_rgf_transmission_f64_noalloc: occupancy query failed");
     // The kernel takes work from a counter, so any grid >= 1 is valid.  On a
     // 148-SM B200 the occupancy grid is 2 blocks per SM at padded order 48
-    // (296 blocks, capped to the fit of 227 at n = 48), 4 at 32 (592, capped
-    // to 511 at n = 32), 6 at 24, 10 at 16 and 16 at 8 (all below the fit).
+    // (296 blocks, capped to the fit of 227 at n = 48: 69 SMs get no second
+    // point), 4 at 32 (592, capped to 511 at n = 32), 6 at 24, 10 at 16 and 16
+    // at 8 (all below the fit).
     const size_t fit = (kNoAllocScratchBytes - kCounterBytes) / per_block;
     if ((size_t)grid > fit) grid = (int)fit;
   }

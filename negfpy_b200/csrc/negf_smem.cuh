@@ -1,6 +1,7 @@
-// One (omega, k) point of block order n <= 48 on one thread block: FP64
-// products on the tensor path and a Gauss-Jordan inverse whose matrix stays in
-// registers, with three matrices in shared memory.
+// Building blocks of one (omega, k) point on one thread block -- FP64 products on
+// the tensor path and a Gauss-Jordan inverse whose matrix stays in registers -- and
+// the kernels of block order n <= 48, with three matrices in shared memory.  The
+// kernels up to order 104 (negf_mid.cuh) use the blocks, too.
 //
 // What bounds these kernels is the FP64 pipe (64 multiply-adds per clock and
 // SM, the same for DMMA and DFMA, which share it) and the latency of the n
@@ -8,7 +9,7 @@
 // through every pivot chain, so several points share an SM: the matrix being
 // inverted and all product results live in registers (each thread owns fixed
 // elements, see Lane), which leaves three matrices per point in shared memory
-// -- 110 KB at n = 48, two points per SM; 28 KB at n = 24, seven.
+// -- 110 KB at n = 48, two points per SM; 31 KB at n = 24, six.
 //
 // Tiles are 8 x 8 (mma.sync m8n8k4, full rate on sm_100a; m16n8k8 is four of
 // them, bit for bit), so orders pad to a multiple of 8 only.
