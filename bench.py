@@ -445,7 +445,7 @@ def grad_vs_forward(torch, n_k=8, n_omega=256, reps=3):
 def uneven_batch(torch, omega_stride=16, oracle_per_system=2):
     """The uneven batch (64 seeded systems, n in {24..192}, 10-60 layers,
     1-256 k, 1024 omegas each) on every ``omega_stride``-th omega of each
-    system: autotuned launch shape and item order, one persistent launch per
+    system: autotuned launch shape and item order, one call of persistent kernels per
     solve replayed from a CUDA graph, FP64 and mixed (FP32 device sweep without
     refinement, FP64 re-solve of failed items).  Reports points/s of both and
     the per-system kappa(300 K) error of the mixed result against FP64."""
@@ -573,7 +573,7 @@ def uneven_batch(torch, omega_stride=16, oracle_per_system=2):
             "kappa_rel_err_median": float(np.nanmedian(errs)) if np.isfinite(errs).any() else None,
             "kappa_err_reference": "the FP64 batch on the same omegas (kappa needs the whole omega grid)",
             "oracle_sample": oracle,
-            "launch": "one persistent kernel per solve (or, in `split`, one per padded-order class), replayed "
+            "launch": "one call of persistent kernels per solve (or, in `split`, per padded-order class), replayed "
                       "from a CUDA graph; launch shape and item order autotuned, per class for the split schedule"}
 
 
